@@ -34,6 +34,7 @@ namespace ix {
 namespace {
 
 constexpr uint32_t POOL_CHUNK = 32;   // paths a warp claims at once: one camera sample per lane
+constexpr uint32_t POOL_QUAD = 4;     // ... of a launch too small for that: one path per group
 constexpr uint32_t POOL_RING = 64;    // prepared camera samples a warp holds
 constexpr uint32_t NO_CHUNK = 0xFFFFFFFFu;
 constexpr unsigned FULL = 0xFFFFFFFFu;
@@ -64,12 +65,12 @@ struct WarpPool {
     PoolJob pending;  // a claimed chunk's job, waiting for the warp to drain
 };
 
-// The warp fills its ring from `chunk` of job `J`: lane l prepares path
-// (chunk - chunk_begin) * 32 + l, sample-major within the job.  Returns the paths added.
-IX_DEV uint32_t pool_fill(WarpPool& wp, const PoolJob& J, uint32_t chunk, uint32_t tail) {
+// The warp fills its ring from `chunk` (of `size` paths) of job `J`: lane l prepares path
+// (chunk - chunk_begin) * size + l, sample-major within the job.  Returns the paths added.
+IX_DEV uint32_t pool_fill(WarpPool& wp, const PoolJob& J, uint32_t chunk, uint32_t size, uint32_t tail) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t first = (chunk - J.chunk_begin) * POOL_CHUNK;
-    const uint32_t n_valid = min(POOL_CHUNK, J.paths - first);
+    const uint32_t first = (chunk - J.chunk_begin) * size;
+    const uint32_t n_valid = min(size, J.paths - first);
     __syncwarp();  // every lane has read the slots this fill may reuse
     if (lane < n_valid) {
         const uint32_t i = first + lane;
@@ -95,10 +96,11 @@ IX_DEV uint32_t pool_fill(WarpPool& wp, const PoolJob& J, uint32_t chunk, uint32
 // The path-pool loop of one warp.  `job_of(chunk, &job)` fills the job a global chunk
 // belongs to and returns its index; `load_planes(job)` returns the job's planes (called
 // with the warp converged and its groups idle).  The k-th claim on `counter` takes chunk
-// k * stride while that is below total_chunks.  Returns the samples this lane dropped.
+// k * stride while that is below total_chunks; a chunk is `size` paths, at most POOL_CHUNK.
+// Returns the samples this lane dropped.
 template <int UNI, class JobOf, class LoadPlanes>
-IX_DEV uint32_t pool_loop(const Group& g, uint32_t* counter, uint32_t total_chunks, uint32_t stride, WarpPool& wp,
-                          JobOf job_of, LoadPlanes load_planes) {
+IX_DEV uint32_t pool_loop(const Group& g, uint32_t* counter, uint32_t total_chunks, uint32_t size, uint32_t stride,
+                          WarpPool& wp, JobOf job_of, LoadPlanes load_planes) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t gi = lane >> 3;
     uint32_t head = 0, tail = 0;  // ring cursors (warp-uniform)
@@ -137,7 +139,7 @@ IX_DEV uint32_t pool_loop(const Group& g, uint32_t* counter, uint32_t total_chun
                     cur_job = pending_job;
                 }
                 if (pending_job == cur_job) {
-                    tail += pool_fill(wp, wp.job, pending, tail);
+                    tail += pool_fill(wp, wp.job, pending, size, tail);
                     pending = NO_CHUNK;
                 }
             }
@@ -202,7 +204,13 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) IX_SFX(pool_trace_kernel)(co
     const Group g = make_group();
     WarpPool& wp = s_pool[threadIdx.x >> 5];
     const uint32_t paths = L.n_pixels * L.spp;
-    const uint32_t total_chunks = (paths + POOL_CHUNK - 1) / POOL_CHUNK;
+    // Chunks of a quad while a resident warp's share is below two chunks of 32 paths: every
+    // warp of a small launch then has its first path at once, and the launch ends evenly.
+    // Kernel time on 4736 warps, chunks of 32 / of 4: 160 x 120 x 1 sample (4 paths a warp)
+    // 518 / 169 us, 256 x 256 x 2 (28) 763 / 490, 256 x 256 x 4 (55) 942 / 809.  Past that the
+    // tail is short next to the launch, and 32 samples prepared at once keep their width.
+    const uint32_t size = paths / (gridDim.x * WARPS) < 2u * POOL_CHUNK ? POOL_QUAD : POOL_CHUNK;
+    const uint32_t total_chunks = (paths + size - 1) / size;
     auto job_of = [&](uint32_t, PoolJob& j) {
         if ((threadIdx.x & 31u) == 0) {
             j.scene = &L.scene;
@@ -220,7 +228,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) IX_SFX(pool_trace_kernel)(co
         return 0;
     };
     auto load_planes = [&](const PoolJob&) { return (const float4*)s_planes; };
-    const uint32_t drops = pool_loop<UNI>(g, L.task_counter, total_chunks, 1u, wp, job_of, load_planes);
+    const uint32_t drops = pool_loop<UNI>(g, L.task_counter, total_chunks, size, 1u, wp, job_of, load_planes);
     if (drops && L.dropped) atomicAdd(L.dropped, (unsigned long long)drops);
 }
 
@@ -272,7 +280,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) IX_SFX(pool_batch_kernel)(co
         }
         return (const float4*)slot;
     };
-    const uint32_t drops = pool_loop<UNI>(g, L.task_counter, L.total_chunks, L.stride, wp, job_of, load_planes);
+    const uint32_t drops = pool_loop<UNI>(g, L.task_counter, L.total_chunks, POOL_CHUNK, L.stride, wp, job_of, load_planes);
     if (drops && L.dropped) atomicAdd(L.dropped, (unsigned long long)drops);
 }
 
