@@ -329,51 +329,19 @@ float d65_host(float lambda) {
     return std::fma(frac, kD65[i0 + 1] - kD65[i0], kD65[i0]) / 100.0f;
 }
 
-// measure_model_width (render_setup/stone_width.rs:27, geometry/stone_metrics/measure.rs):
-// the narrower horizontal extent (x or z) of the solid's vertices, in f64.  A vertex is
-// any point where three planes meet and no plane is violated by more than 1e-9.
-double solid_width(const float* planes, uint32_t n) {
-    std::vector<std::array<double, 4>> pl;  // n.x <= m with m = -d
+// The distinct planes of a stone in f64, n.x <= m with m = -d, appended to `out` (4 per plane).
+uint32_t append_distinct_planes(const float* planes, uint32_t n, std::vector<double>* out) {
+    const size_t first = out->size();
     for (uint32_t i = 0; i < n; ++i) {
-        std::array<double, 4> p{planes[4 * i], planes[4 * i + 1], planes[4 * i + 2], -(double)planes[4 * i + 3]};
+        const double p[4] = {planes[4 * i], planes[4 * i + 1], planes[4 * i + 2], -(double)planes[4 * i + 3]};
         bool same = false;
-        for (const auto& q : pl)
-            if (p[0] * q[0] + p[1] * q[1] + p[2] * q[2] > 1.0 - 1e-12 && std::fabs(p[3] - q[3]) < 1e-9) same = true;
-        if (!same) pl.push_back(p);
+        for (size_t q = first; q < out->size(); q += 4) {
+            const double* o = out->data() + q;
+            if (p[0] * o[0] + p[1] * o[1] + p[2] * o[2] > 1.0 - 1e-12 && std::fabs(p[3] - o[3]) < 1e-9) same = true;
+        }
+        if (!same) out->insert(out->end(), p, p + 4);
     }
-    const size_t m = pl.size();
-    double lo[2] = {INFINITY, INFINITY}, hi[2] = {-INFINITY, -INFINITY};
-    size_t found = 0;
-    auto cr = [](const std::array<double, 4>& a, const std::array<double, 4>& b, double o[3]) {
-        o[0] = a[1] * b[2] - a[2] * b[1];
-        o[1] = a[2] * b[0] - a[0] * b[2];
-        o[2] = a[0] * b[1] - a[1] * b[0];
-    };
-    for (size_t i = 0; i < m; ++i)
-        for (size_t j = i + 1; j < m; ++j)
-            for (size_t k = j + 1; k < m; ++k) {
-                double jk[3], ki[3], ij[3];
-                cr(pl[j], pl[k], jk);
-                double det = pl[i][0] * jk[0] + pl[i][1] * jk[1] + pl[i][2] * jk[2];
-                if (std::fabs(det) < 1e-12) continue;
-                cr(pl[k], pl[i], ki);
-                cr(pl[i], pl[j], ij);
-                double v[3];
-                for (int a = 0; a < 3; ++a) v[a] = (pl[i][3] * jk[a] + pl[j][3] * ki[a] + pl[k][3] * ij[a]) / det;
-                if (!std::isfinite(v[0]) || !std::isfinite(v[1]) || !std::isfinite(v[2])) continue;
-                bool inside = true;
-                for (size_t q = 0; inside && q < m; ++q)
-                    inside = pl[q][0] * v[0] + pl[q][1] * v[1] + pl[q][2] * v[2] - pl[q][3] <= 1e-9;
-                if (!inside) continue;
-                ++found;
-                lo[0] = std::min(lo[0], v[0]);
-                hi[0] = std::max(hi[0], v[0]);
-                lo[1] = std::min(lo[1], v[2]);
-                hi[1] = std::max(hi[1], v[2]);
-            }
-    if (found < 4) return NAN;
-    const double dx = hi[0] - lo[0], dz = hi[1] - lo[1];
-    return dx <= dz ? dx : dz;
+    return (uint32_t)((out->size() - first) / 4);
 }
 
 // head_shadow_cone_cos (visibility.rs:16).
@@ -503,6 +471,7 @@ void ix_backend_destroy(ix_backend* b) {
     cudaFree(b->d_finishes);
     cudaFree(b->d_tools);
     cudaFree(b->d_acc);
+    cudaFree(b->d_metrics);
     display_state_free(b->display);
     radiance_state_free(b->radiance);
     if (b->h_attr_map) cudaFreeHost(b->h_attr_map);
@@ -1511,11 +1480,15 @@ int ix_evaluate_gem_optical_metrics_batch(ix_backend* b, const ix_metrics_stone*
     L.n_poses = n_poses;
     std::vector<float> planes;
     std::vector<ix::MetricsStoneDev> dstones(n_stones);
+    std::vector<double> wplanes;
+    std::vector<ix::WidthStoneDev> wstones(n_stones);
+    const ix::ExtentsDev none{{~0ull, ~0ull}, {0ull, 0ull}, 0u, 0u};
+    const std::vector<ix::ExtentsDev> extents(n_stones, none);
     for (uint32_t s = 0; s < n_stones; ++s) {
         dstones[s].plane_offset = (uint32_t)(planes.size() / 4);
         dstones[s].n_planes = stones[s].n_planes;
-        const double w = solid_width(stones[s].planes, stones[s].n_planes);
-        dstones[s].half_width = (std::isfinite(w) && w > 0.0) ? (float)(w * 0.5) : 1.0f;
+        wstones[s].first = (uint32_t)(wplanes.size() / 4);
+        wstones[s].n_planes = append_distinct_planes(stones[s].planes, stones[s].n_planes, &wplanes);
         dstones[s].dispersion = stones[s].dispersion;
         planes.insert(planes.end(), stones[s].planes, stones[s].planes + 4 * (size_t)stones[s].n_planes);
     }
@@ -1525,7 +1498,8 @@ int ix_evaluate_gem_optical_metrics_batch(ix_backend* b, const ix_metrics_stone*
     std::vector<ix::MetricsPoseDev> dposes(n_poses);
     for (uint32_t p = 0; p < n_poses; ++p) {
         dposes[p].stone = poses[p].stone;
-        for (int k = 0; k < 6; ++k) {
+        const int n_bases = L.want_fire ? 6 : 1;  // the jittered poses' rays are traced with fire only
+        for (int k = 0; k < n_bases; ++k) {
             ix_camera cam;
             const float yaw = k == 0 ? poses[p].cam_yaw : poses[p].cam_yaw + to_radians(kOffsets[k - 1]);
             ix_camera_new(yaw, poses[p].cam_pitch, 1.0f, 42.0f, &cam);
@@ -1536,42 +1510,46 @@ int ix_evaluate_gem_optical_metrics_batch(ix_backend* b, const ix_metrics_stone*
     }
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
-    float *d_planes = nullptr, *d_out = nullptr;
-    ix::MetricsStoneDev* d_stones = nullptr;
-    ix::MetricsPoseDev* d_poses = nullptr;
-    bool ok = cudaMalloc((void**)&d_planes, planes.size() * sizeof(float)) == cudaSuccess &&
-              cudaMalloc((void**)&d_stones, n_stones * sizeof(ix::MetricsStoneDev)) == cudaSuccess &&
-              cudaMalloc((void**)&d_poses, n_poses * sizeof(ix::MetricsPoseDev)) == cudaSuccess &&
-              cudaMalloc((void**)&d_out, (size_t)n_poses * 5 * sizeof(float)) == cudaSuccess;
-    ok = ok && cudaMemcpyAsync(d_planes, planes.data(), planes.size() * sizeof(float), cudaMemcpyHostToDevice,
-                               b->stream) == cudaSuccess &&
-         cudaMemcpyAsync(d_stones, dstones.data(), n_stones * sizeof(ix::MetricsStoneDev), cudaMemcpyHostToDevice,
-                         b->stream) == cudaSuccess &&
-         cudaMemcpyAsync(d_poses, dposes.data(), n_poses * sizeof(ix::MetricsPoseDev), cudaMemcpyHostToDevice,
-                         b->stream) == cudaSuccess;
-    if (ok) {
-        L.planes = reinterpret_cast<const float4*>(d_planes);
-        L.stones = d_stones;
-        L.poses = d_poses;
-        L.out = d_out;
-        cudaError_t e = b->precision == IX_PRECISION_EXACT ? ix::launch_metrics_exact(L, b->stream)
-                                                           : ix::launch_metrics_fast(L, b->stream);
-        ok = !fail(b, e, "metrics launch");
-        std::vector<float> host((size_t)n_poses * 5);
-        ok = ok && !fail(b, cudaMemcpyAsync(host.data(), d_out, host.size() * sizeof(float), cudaMemcpyDeviceToHost,
-                                            b->stream), "metrics download");
-        ok = ok && !fail(b, cudaStreamSynchronize(b->stream), "metrics sync");
-        if (ok)
-            for (uint32_t p = 0; p < n_poses; ++p)
-                out[p] = ix_gem_metrics{host[5 * p], host[5 * p + 1], host[5 * p + 2], host[5 * p + 3],
-                                        host[5 * p + 4]};
-    } else {
-        fail(b, cudaGetLastError(), "metrics buffers");
-    }
-    cudaFree(d_planes);
-    cudaFree(d_stones);
-    cudaFree(d_poses);
-    cudaFree(d_out);
+    // One buffer and one upload, each part 16-byte aligned; the results after them.
+    std::vector<uint8_t> up;
+    auto part = [&](const void* p, size_t bytes) {
+        const size_t at = up.size();
+        up.resize((at + bytes + 15) & ~(size_t)15);
+        std::memcpy(up.data() + at, p, bytes);
+        return at;
+    };
+    const size_t at_planes = part(planes.data(), planes.size() * sizeof(float));
+    const size_t at_stones = part(dstones.data(), n_stones * sizeof(ix::MetricsStoneDev));
+    const size_t at_wplanes = part(wplanes.data(), wplanes.size() * sizeof(double));
+    const size_t at_wstones = part(wstones.data(), n_stones * sizeof(ix::WidthStoneDev));
+    const size_t at_extents = part(extents.data(), n_stones * sizeof(ix::ExtentsDev));
+    const size_t at_poses = part(dposes.data(), n_poses * sizeof(ix::MetricsPoseDev));
+    const size_t at_out = up.size();
+    if (fail(b, grow_device(&b->d_metrics, &b->metrics_cap, at_out + (size_t)n_poses * 5 * sizeof(float)),
+             "metrics buffers") ||
+        fail(b, cudaMemcpyAsync(b->d_metrics, up.data(), up.size(), cudaMemcpyHostToDevice, b->stream),
+             "metrics upload"))
+        return IX_DECLINED;
+    uint8_t* const d = b->d_metrics;
+    const ix::WidthLaunch W{reinterpret_cast<const double*>(d + at_wplanes),
+                            reinterpret_cast<const ix::WidthStoneDev*>(d + at_wstones),
+                            reinterpret_cast<ix::ExtentsDev*>(d + at_extents), n_stones};
+    if (fail(b, ix::launch_stone_extents(W, b->stream), "stone extents launch")) return IX_DECLINED;
+    L.planes = reinterpret_cast<const float4*>(d + at_planes);
+    L.stones = reinterpret_cast<const ix::MetricsStoneDev*>(d + at_stones);
+    L.extents = W.out;
+    L.poses = reinterpret_cast<const ix::MetricsPoseDev*>(d + at_poses);
+    L.out = reinterpret_cast<float*>(d + at_out);
+    cudaError_t e = b->precision == IX_PRECISION_EXACT ? ix::launch_metrics_exact(L, b->stream)
+                                                       : ix::launch_metrics_fast(L, b->stream);
+    bool ok = !fail(b, e, "metrics launch");
+    std::vector<float> host((size_t)n_poses * 5);
+    ok = ok && !fail(b, cudaMemcpyAsync(host.data(), L.out, host.size() * sizeof(float), cudaMemcpyDeviceToHost,
+                                        b->stream), "metrics download");
+    ok = ok && !fail(b, cudaStreamSynchronize(b->stream), "metrics sync");
+    if (ok)
+        for (uint32_t p = 0; p < n_poses; ++p)
+            out[p] = ix_gem_metrics{host[5 * p], host[5 * p + 1], host[5 * p + 2], host[5 * p + 3], host[5 * p + 4]};
     return ok ? IX_DONE : IX_DECLINED;
 }
 
@@ -1657,9 +1635,9 @@ int ix_debug_check(ix_backend* b, const ix_scene* scene, int32_t fn, uint32_t n,
     if (scene->n_planes > IX_MAX_PLANES) return -1;
     // 32-bit words each check function reads from / writes to a row (ix::CheckFn order):
     // rows narrower than that are refused before anything reaches the device.
-    static const uint8_t kIn[] = {2, 1, 1, 1, 1, 1, 3, 7, 7, 6, 2, 2, 1, 8, 14, 7, 4, 9};
-    static const uint8_t kOut[] = {4, 8, 1, 3, 1, 1, 1, 6, 1, 2, 4, 6, 1, 4, 7, 13, 1, 24};
-    static_assert(sizeof(kIn) == ix::CHECK_BIAXIAL + 1 && sizeof(kOut) == sizeof(kIn), "check table");
+    static const uint8_t kIn[] = {2, 1, 1, 1, 1, 1, 3, 7, 7, 6, 2, 2, 1, 8, 14, 7, 4, 9, 7};
+    static const uint8_t kOut[] = {4, 8, 1, 3, 1, 1, 1, 6, 1, 2, 4, 6, 1, 4, 7, 13, 1, 24, 2};
+    static_assert(sizeof(kIn) == ix::CHECK_INTERIOR_HIT + 1 && sizeof(kOut) == sizeof(kIn), "check table");
     if (fn < 0 || fn >= (int32_t)sizeof(kIn) || in_stride < kIn[fn] || out_stride < kOut[fn]) return -1;
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return -1;

@@ -59,6 +59,9 @@ struct ix_backend {
     // Fixed-point per-pixel sums of the path-pool kernels (FIXED_WORDS per pixel of a launch).
     unsigned long long* d_acc = nullptr;
     size_t acc_cap = 0;
+    // The metrics call's stones, poses and results.
+    uint8_t* d_metrics = nullptr;
+    size_t metrics_cap = 0;
     int sm_count = 0;
     // Kernel variant (budget + 3 * shape, ix_launch.h) of single-scene calls.
     uint32_t variant = 0;

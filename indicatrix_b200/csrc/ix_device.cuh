@@ -667,18 +667,31 @@ IX_DEV float exit_lighting_threshold(const ix_environment& env, float spec, floa
         const V3 d = v3(dirs[i][0], dirs[i][1], dirs[i][2]);
         s_rad[i] = exit_radiance<SCORE>(env, spec, d);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 1; i < 96; ++i) {  // insertion sort, ascending
-            const float v = s_rad[i];
-            int j = i - 1;
-            while (j >= 0 && s_rad[j] > v) {
-                s_rad[j + 1] = s_rad[j];
-                --j;
+    // The 49th smallest: the radiance that 48 others precede (equal ones in index order),
+    // found by a thread per radiance; sorting the 96 on one thread takes 35 us and is left for
+    // radiances that do not compare.
+    bool nan = false;
+    for (int i = threadIdx.x; i < 96; i += blockDim.x) nan = nan || isnan(s_rad[i]);
+    if (__syncthreads_or(nan)) {
+        if (threadIdx.x == 0) {
+            for (int i = 1; i < 96; ++i) {  // insertion sort, ascending
+                const float v = s_rad[i];
+                int j = i - 1;
+                while (j >= 0 && s_rad[j] > v) {
+                    s_rad[j + 1] = s_rad[j];
+                    --j;
+                }
+                s_rad[j + 1] = v;
             }
-            s_rad[j + 1] = v;
+            *s_threshold = fmaxf(s_rad[48] * factor, 1.17549435e-38f);
         }
-        *s_threshold = fmaxf(s_rad[48] * factor, 1.17549435e-38f);
+    } else {
+        for (int i = threadIdx.x; i < 96; i += blockDim.x) {
+            const float v = s_rad[i];
+            int before = 0;
+            for (int j = 0; j < 96; ++j) before += (s_rad[j] < v || (s_rad[j] == v && j < i)) ? 1 : 0;
+            if (before == 48) *s_threshold = fmaxf(v * factor, 1.17549435e-38f);
+        }
     }
     __syncthreads();
     return *s_threshold;

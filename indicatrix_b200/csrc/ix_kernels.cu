@@ -20,6 +20,7 @@
 // The batch kernel runs the same task loop over many scenes (stones x tilts) in one
 // launch; each warp keeps the planes of the scene it is working on in its own
 // shared-memory slot.
+#include "ix_interior.cuh"
 #include "ix_launch.h"
 #include "ix_transport.cuh"
 
@@ -407,6 +408,27 @@ __global__ void __launch_bounds__(128) IX_SFX(check_trace_kernel)(const __grid_c
     }
 }
 
+// The slab scans of a converged warp, a group per input row.
+__global__ void __launch_bounds__(128) IX_SFX(check_scan_kernel)(const __grid_constant__ CheckLaunch L) {
+    __shared__ float4 s_rows[IX_MAX_PLANES], s_pairs[PLANE_PAIR_VECS];
+    const int n = (int)L.scene.n_planes;
+    stage_planes(reinterpret_cast<const float4*>(L.scene.planes), n, s_rows, s_pairs, (int)threadIdx.x, 128);
+    __syncthreads();
+    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const uint32_t* in = L.in + (size_t)min(row, L.n - 1u) * L.in_stride;
+    const V3 o = v3(__uint_as_float(in[0]), __uint_as_float(in[1]), __uint_as_float(in[2]));
+    const V3 d = v3(__uint_as_float(in[3]), __uint_as_float(in[4]), __uint_as_float(in[5]));
+    Hit h;
+    const bool decided = warp_interior_hit(s_rows, s_pairs, n, o, d, h);
+    const Hit e = warp_exact_hit(s_rows, n, o, d);
+    if (!decided || in[6] == 0) h = e;
+    if (row < L.n && (threadIdx.x & 7u) == 0) {
+        uint32_t* out = L.out + (size_t)row * L.out_stride;
+        out[0] = __float_as_uint(h.t);
+        out[1] = __float_as_uint((float)h.facet);
+    }
+}
+
 // One reference function per thread, for the per-function parity checks.
 __global__ void IX_SFX(check_kernel)(const __grid_constant__ CheckLaunch L) {
     __shared__ float4 s_planes[IX_MAX_PLANES];
@@ -677,7 +699,9 @@ cudaError_t IX_SFX(launch_check)(const CheckLaunch& l, cudaStream_t stream) {
     if (l.scene.n_planes > IX_MAX_PLANES) return cudaErrorInvalidValue;
     if (l.n == 0) return cudaSuccess;
     const int threads = 128;
-    if (l.fn == CHECK_TRACE || l.fn == CHECK_TRACE_RAY) {
+    if (l.fn == CHECK_INTERIOR_HIT) {
+        IX_SFX(check_scan_kernel)<<<(int)((l.n * 8ull + threads - 1) / threads), threads, 0, stream>>>(l);
+    } else if (l.fn == CHECK_TRACE || l.fn == CHECK_TRACE_RAY) {
         const int blocks = (int)((l.n * 8ull + threads - 1) / threads);
         switch (transport_class(l.flags)) {
             case TRANSPORT_EXTENDED: IX_SFX(check_trace_kernel)<TRANSPORT_EXTENDED><<<blocks, threads, 0, stream>>>(l); break;

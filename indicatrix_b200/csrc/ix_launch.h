@@ -230,6 +230,8 @@ enum CheckFn {
                               // (slow xyz, fast xyz), mode_poynting_dir (slow, fast),
                               // resolve_entry_mode (slow n, dir xyz, fast n, dir xyz), assigned-
                               // mode alpha of the trichroic tensor (mode B, mode A)
+    CHECK_INTERIOR_HIT = 18,  // in: origin xyz, dir xyz, interior (0 / 1)  out: t, facet (as float), by
+                              // the 8-lane exact scan or by the interior scan where it decides
 };
 
 struct CheckLaunch {
@@ -247,9 +249,24 @@ struct CheckLaunch {
 struct MetricsStoneDev {
     uint32_t plane_offset;  // first float4 of the stone in `planes`
     uint32_t n_planes;
-    float half_width;       // girdle half-width (fan.rs:34), measured on the host in f64
     ix_dispersion dispersion;
 };
+// A stone's distinct planes in f64 (n.x <= m: the normal and m), for its width.
+struct WidthStoneDev {
+    uint32_t first, n_planes;
+};
+// The solid's x and z extents as order-preserving integers, and its vertex count.
+struct ExtentsDev {
+    unsigned long long lo[2], hi[2];
+    uint32_t found, pad;
+};
+struct WidthLaunch {
+    const double* planes;         // device, 4 per plane
+    const WidthStoneDev* stones;  // device
+    ExtentsDev* out;              // device, one per stone: lo all ones, hi and found zero
+    uint32_t n_stones;
+};
+cudaError_t launch_stone_extents(const WidthLaunch& l, cudaStream_t stream);
 struct MetricsPoseDev {
     uint32_t stone;
     float basis[6][9];  // forward, right, up of the pose and of its 5 yaw-jittered poses
@@ -257,6 +274,7 @@ struct MetricsPoseDev {
 struct MetricsLaunch {
     const float4* planes;          // device
     const MetricsStoneDev* stones;  // device
+    const ExtentsDev* extents;      // device, per stone (the girdle half-width, fan.rs:34)
     const MetricsPoseDev* poses;    // device
     uint32_t n_poses;
     uint32_t want_fire;             // fire and scintillation rays traced
