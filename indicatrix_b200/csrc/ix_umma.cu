@@ -6,16 +6,16 @@
 //   * all 256 threads stage 64-wide K slices of A and B into shared memory in the
 //     tensor cores' K-major, unswizzled canonical layout (8-row x 16-byte core matrices),
 //     zero-filling past the matrix edges, STAGES slices deep: rows contiguous along K go
-//     by 16-byte cp.async (in flight while earlier slices multiply), transposed views
-//     element by element;
+//     by 16-byte cp.async (in flight while earlier slices multiply), transposed views by
+//     16-byte loads along the rows, two k at a time, turned in registers (stage_turned);
 //   * one thread issues the slice's four tcgen05.mma (M 128, N NT, K 16 each) with shared
 //     memory descriptors and commits them to the stage's mbarrier, which the threads wait
 //     on before they refill that stage;
 //   * the accumulator lives in TMEM (NT columns, allocated by warp 0); after the last
 //     commit each warp reads its lane quadrant's rows (half of the columns) with tcgen05.ld,
-//     transposes them through shared memory and applies the fused epilogue with coalesced
-//     stores: store,
-//     bias + SiLU (forward), or the SiLU derivative (backward).
+//     transposes them through shared memory and applies the fused epilogue -- store, bias +
+//     SiLU (forward), or the SiLU derivative (backward) -- four columns a lane with 16-byte
+//     accesses where the output allows it.
 // Tall-K products with few output tiles (weight gradients: K = the batch) split K over
 // blockIdx.z into f32 partials that a second kernel sums in split order, so results do
 // not depend on scheduling.
@@ -116,14 +116,48 @@ __device__ __forceinline__ float silu_grad(float z) {
     return s * (1.0f + z * (1.0f - s));
 }
 
+// The transposed view of an operand (rows adjacent in memory, 16-byte aligned columns, every
+// row of the tile and k of the slice inside the matrix): a thread reads 8 rows of two
+// neighbouring k and writes eight 4-byte pairs.  The pairs of 8 threads with neighbouring
+// row octets fall on the same four banks, so each thread starts at another of its eight rows
+// and the warp's stores never conflict.  The weight gradient 256 x 256 x 4096 took 75 us with
+// 2-byte loads and stores, 24 us so.
+template <int R>
+__device__ void stage_turned(uint8_t* stage, const __nv_bfloat16* g, int64_t ks, uint32_t r0, uint32_t k0) {
+    constexpr uint32_t OCTETS = R / 8;
+    for (uint32_t idx = threadIdx.x; idx < OCTETS * (BK / 2); idx += THREADS) {
+        const uint32_t oct = idx % OCTETS, kp = idx / OCTETS;
+        const __nv_bfloat16* p = g + (int64_t)(k0 + 2 * kp) * ks + r0 + oct * 8;
+        const uint4 lo = *reinterpret_cast<const uint4*>(p), hi = *reinterpret_cast<const uint4*>(p + ks);
+        const uint32_t a[4] = {lo.x, lo.y, lo.z, lo.w}, b[4] = {hi.x, hi.y, hi.z, hi.w};
+        uint32_t pair[8];  // rows 0 .. 7: k in the low half, k + 1 in the high
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            pair[2 * j] = __byte_perm(a[j], b[j], 0x5410);
+            pair[2 * j + 1] = __byte_perm(a[j], b[j], 0x7632);
+        }
+        uint8_t* dst = stage + ((kp / 4) * OCTETS + oct) * 128 + (kp % 4) * 4;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t row = ((uint32_t)j + oct) & 7u;
+            uint32_t v = pair[0];
+#pragma unroll
+            for (int q = 1; q < 8; ++q) v = row == (uint32_t)q ? pair[q] : v;
+            *reinterpret_cast<uint32_t*>(dst + row * 16) = v;
+        }
+    }
+}
+
 // Stages rows [r0, r0 + R) x k [k0, k0 + BK) of an operand into `stage` in the canonical
 // layout -- element (r, k) at ((k / 8) * (R / 8) + r / 8) * 128 + (r % 8) * 16 + (k % 8) * 2
 // bytes -- with zeros at rows >= rows and k >= k_end.
 template <int R>
 __device__ void stage_tile(uint8_t* stage, const __nv_bfloat16* g, int64_t rs, int64_t ks, uint32_t r0, uint32_t rows,
-                           uint32_t k0, uint32_t k_end, bool vec) {
+                           uint32_t k0, uint32_t k_end, bool vec, bool turned) {
     const uint32_t tid = threadIdx.x;
-    if (vec) {
+    if (turned && r0 + R <= rows && k0 + BK <= k_end) {
+        stage_turned<R>(stage, g, ks, r0, k0);
+    } else if (vec) {
         // 16-byte vectors along K (ks == 1, rows 16-byte aligned); consecutive threads
         // take consecutive rows of one 8-wide K chunk.
         // cp.async with a source size: bytes past it (the matrix's edge) are zero-filled;
@@ -166,6 +200,8 @@ __global__ void __launch_bounds__(THREADS) umma_gemm_kernel(const __grid_constan
     const uint32_t k_end = min(P.k, k_begin + P.k_split);
     const bool a_vec = P.a_ks == 1 && (P.a_rs % 8) == 0 && (((uintptr_t)P.a) & 15u) == 0;
     const bool b_vec = P.b_ks == 1 && (P.b_rs % 8) == 0 && (((uintptr_t)P.b) & 15u) == 0;
+    const bool a_turned = P.a_rs == 1 && (P.a_ks % 8) == 0 && (((uintptr_t)P.a) & 15u) == 0;
+    const bool b_turned = P.b_rs == 1 && (P.b_ks % 8) == 0 && (((uintptr_t)P.b) & 15u) == 0;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_taddr)),
@@ -187,8 +223,8 @@ __global__ void __launch_bounds__(THREADS) umma_gemm_kernel(const __grid_constan
     auto b_slot = [&](uint32_t slot) { return smem + STAGES * A_STAGE + slot * B_STAGE; };
     auto load = [&](uint32_t slice) {
         const uint32_t slot = slice % STAGES, k0 = k_begin + slice * BK;
-        stage_tile<TM>(a_slot(slot), P.a, P.a_rs, P.a_ks, r0, P.m, k0, k_end, a_vec);
-        stage_tile<NT>(b_slot(slot), P.b, P.b_rs, P.b_ks, c0, P.n, k0, k_end, b_vec);
+        stage_tile<TM>(a_slot(slot), P.a, P.a_rs, P.a_ks, r0, P.m, k0, k_end, a_vec, a_turned);
+        stage_tile<NT>(b_slot(slot), P.b, P.b_rs, P.b_ks, c0, P.n, k0, k_end, b_vec, b_turned);
     };
     // Prologue: slices 0 .. STAGES - 2 in flight.  Every iteration commits one cp.async
     // group (possibly empty), so "all but the newest STAGES - 2 groups done" always means
@@ -272,21 +308,60 @@ __global__ void __launch_bounds__(THREADS) umma_gemm_kernel(const __grid_constan
         }
         __syncwarp();
         float* out_f32 = P.out_f32 ? P.out_f32 + (size_t)blockIdx.z * P.m * P.ldo : nullptr;
-        for (int r = 0; r < 32; ++r) {
-            const uint32_t row = r0 + quad * 32 + r;
-            if (row >= P.m) break;
-            for (int c = lane; c < HW; c += 32) {
-                const uint32_t col = c0 + half * HW + c;
-                if (col >= P.n) break;
-                float x = stage[r * (HW + 1) + c];
+        auto element = [&](float x, float bias, float zprev, float& z) {
+            if (P.epi == EPI_BIAS_ACT) {
+                if (P.bias) x += bias;
+                z = x;
+                if (P.act) x = silu(x);
+            } else if (P.epi == EPI_SILU_GRAD) {
+                x *= silu_grad(zprev);
+            }
+            return x;
+        };
+        const uint32_t cbase = c0 + half * HW;
+        // Four columns a lane where every row of the output starts on a 16-byte boundary and
+        // the tile's columns are all inside: 4096 x 256 x 256 with bias and SiLU 17.5 -> 14.5 us,
+        // its backward form 32 -> 16 (with the turned staging).
+        auto aligned = [](const void* p, uint32_t bytes) { return (((uintptr_t)p) & (bytes - 1u)) == 0; };
+        const bool wide = P.ldo % 4 == 0 && c0 + NT <= P.n && aligned(out_f32, 16) && aligned(P.out_bf16, 8) &&
+                          aligned(P.out_z, 16) && aligned(P.zprev, 16) && aligned(P.bias, 16);
+        if (wide) {
+            constexpr int QUADS = HW / 4;
+            for (int i = (int)lane; i < 32 * QUADS; i += 32) {
+                const int r = i / QUADS, c = (i % QUADS) * 4;
+                const uint32_t row = r0 + quad * 32 + r, col = cbase + c;
+                if (row >= P.m) continue;
                 const size_t o = (size_t)row * P.ldo + col;
-                if (P.epi == EPI_BIAS_ACT) {
-                    if (P.bias) x += P.bias[col];
-                    if (P.out_z) P.out_z[o] = x;
-                    if (P.act) x = silu(x);
-                } else if (P.epi == EPI_SILU_GRAD) {
-                    x *= silu_grad(P.zprev[o]);
+                const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                const float4 b4 = P.epi == EPI_BIAS_ACT && P.bias ? *reinterpret_cast<const float4*>(P.bias + col) : none;
+                const float4 p4 = P.epi == EPI_SILU_GRAD ? *reinterpret_cast<const float4*>(P.zprev + o) : none;
+                const float* v = stage + r * (HW + 1) + c;
+                float4 z = none, x;
+                x.x = element(v[0], b4.x, p4.x, z.x);
+                x.y = element(v[1], b4.y, p4.y, z.y);
+                x.z = element(v[2], b4.z, p4.z, z.z);
+                x.w = element(v[3], b4.w, p4.w, z.w);
+                if (P.epi == EPI_BIAS_ACT && P.out_z) *reinterpret_cast<float4*>(P.out_z + o) = z;
+                if (out_f32) *reinterpret_cast<float4*>(out_f32 + o) = x;
+                if (P.out_bf16) {
+                    __nv_bfloat162 h[2];
+                    h[0].x = __float2bfloat16_rn(x.x);
+                    h[0].y = __float2bfloat16_rn(x.y);
+                    h[1].x = __float2bfloat16_rn(x.z);
+                    h[1].y = __float2bfloat16_rn(x.w);
+                    *reinterpret_cast<uint2*>(P.out_bf16 + o) = *reinterpret_cast<const uint2*>(h);
                 }
+            }
+        } else {
+            for (int i = (int)lane; i < 32 * HW; i += 32) {
+                const int r = i / HW, c = i % HW;
+                const uint32_t row = r0 + quad * 32 + r, col = cbase + c;
+                if (row >= P.m || col >= P.n) continue;
+                const size_t o = (size_t)row * P.ldo + col;
+                float z = 0.0f;
+                const float x = element(stage[r * (HW + 1) + c], P.epi == EPI_BIAS_ACT && P.bias ? P.bias[col] : 0.0f,
+                                        P.epi == EPI_SILU_GRAD ? P.zprev[o] : 0.0f, z);
+                if (P.epi == EPI_BIAS_ACT && P.out_z) P.out_z[o] = z;
                 if (out_f32) out_f32[o] = x;
                 if (P.out_bf16) P.out_bf16[o] = __float2bfloat16_rn(x);
             }
