@@ -23,7 +23,6 @@ namespace ix {
 // about 10 instructions a plane and no branch, against 20 to 30 of the exact scan, whose
 // lanes divide under a branch.  Padding planes (0, 0, 0, -1e30) have u = 0.
 // ------------------------------------------------------------------------------------
-constexpr unsigned WARP_MASK = 0xFFFFFFFFu;
 constexpr int PAIR_WORDS = 8;  // x, x', y, y', z, z', w, w'
 constexpr int PLANE_PAIR_VECS = IX_MAX_PLANES / 2 * PAIR_WORDS / 4;  // float4s of a full set
 static_assert(IX_MAX_PLANES <= 128, "7 index bits");
@@ -136,7 +135,7 @@ IX_DEV bool warp_interior_hit(const float4* __restrict__ rows, const float4* __r
 }
 // The exact scan of four rays (group_intersect under the full mask).
 IX_DEV Hit warp_exact_hit(const float4* __restrict__ rows, int n, V3 o, V3 d) {
-    return group_intersect(Group{WARP_MASK, (int)(threadIdx.x & 7u)}, rows, n, o, d);
+    return group_intersect(warp_group(), rows, n, o, d);
 }
 
 }  // namespace ix

@@ -112,6 +112,7 @@ IX_DEV uint32_t pool_loop(const Group& g, uint32_t* counter, uint32_t total_chun
     uint32_t row = 0;   // ... and its accumulator row
     uint32_t drops = 0;
     LanePath P;
+    P.o = P.d = v3(0.0f, 0.0f, 0.0f);
     for (;;) {
         const unsigned idle = __ballot_sync(FULL, !busy) & 0x01010101u;
         const uint32_t n_idle = __popc(idle);
@@ -157,8 +158,41 @@ IX_DEV uint32_t pool_loop(const Group& g, uint32_t* counter, uint32_t total_chun
             }
         }
         head += min(n_idle, avail);
-        if (!busy && !fresh) continue;
         const PoolJob& J = wp.job;
+        if constexpr (UNI == TRANSPORT_ISOTROPIC) {
+            if (n_idle == 4 && avail == 0) continue;  // no path, and no job's planes yet
+            const DevScene S = make_scene(*J.scene, J.flags);
+            if (fresh) {
+                const PoolEntry& e = wp.e[slot];
+                row = e.row;
+                const Ray r{load3(S.s.camera.origin), v3(e.d[0], e.d[1], e.d[2])};
+                group_init_ray<UNI>(g, P, S, r, e.seed, e.hero);
+                busy = true;
+            }
+            __syncwarp();
+            // The scan and the colour sum with the warp converged; a group without a path scans
+            // what its last one left.
+            Hit hit = group_intersect(warp_group(), planes, (int)S.s.n_planes, P.o, P.d);
+            float esc = 0.0f;
+            int r = BOUNCE_CONTINUE;
+            bool done = false;
+            if (busy) {
+                const uint32_t max_bounces = S.s.max_bounces;
+                if (!P.inside && P.has_prev && leaves_stone_through(planes, P.facet, P.o, P.d)) hit.facet = -1;
+                r = P.bounce >= max_bounces ? (int)BOUNCE_KILLED : group_bounce_at(g, P, S, planes, hit, esc);
+                done = r != BOUNCE_CONTINUE || P.bounce >= max_bounces;
+            }
+            if (__any_sync(FULL, done)) {
+                // The path finished (escaped, roulette, or reached the bounce cap).
+                const V3 xyz = group_finish<UNI>(warp_group(), P, S, r == BOUNCE_ESCAPED, esc);
+                if (done) {
+                    drops += add_sample_fixed(g, J.acc + (size_t)row * FIXED_WORDS, xyz);
+                    busy = false;
+                }
+            }
+            continue;
+        }
+        if (!busy && !fresh) continue;
         const DevScene S = make_scene(*J.scene, J.flags);
         if (fresh) {
             const PoolEntry& e = wp.e[slot];

@@ -55,6 +55,10 @@ IX_DEV Group make_group() {
     const int lane = (int)(threadIdx.x & 31u);
     return Group{0xFFu << (lane & ~7), lane & 7};
 }
+// Four groups of a converged warp: a shuffle under this constant mask is one instruction,
+// where each group's own mask repeats it per group and carries about 290 bytes of code.
+constexpr unsigned WARP_MASK = 0xFFFFFFFFu;
+IX_DEV Group warp_group() { return Group{WARP_MASK, (int)(threadIdx.x & 7u)}; }
 IX_DEV float gshfl(const Group& g, float v, int src) { return __shfl_sync(g.mask, v, src, 8); }
 IX_DEV int gshfl(const Group& g, int v, int src) { return __shfl_sync(g.mask, v, src, 8); }
 IX_DEV float gxor(const Group& g, float v, int m) { return __shfl_xor_sync(g.mask, v, m, 8); }
@@ -860,10 +864,8 @@ struct BounceGeom {
 
 // Returns BOUNCE_ESCAPED (esc set) or BOUNCE_CONTINUE with P.facet the hit facet and `t`
 // its distance.
-IX_DEV int bounce_hit(const Group& g, LanePath& P, const DevScene& S, const float4* __restrict__ planes, float& esc,
-                      float& t) {
+IX_DEV int bounce_at(LanePath& P, const DevScene& S, const float4* __restrict__ planes, Hit hit, float& esc, float& t) {
     const ix_scene& sc = S.s;
-    Hit hit = group_next_hit(g, P, planes, (int)sc.n_planes);
     if (hit.facet < 0) {
         esc = fmaf(intensity(P.st), lane_environment(sc.environment, P.d, P.observer, P.lambda), 0.0f);
         return BOUNCE_ESCAPED;
@@ -879,6 +881,11 @@ IX_DEV int bounce_hit(const Group& g, LanePath& P, const DevScene& S, const floa
     // apply_interior_segment (transport/inner.rs:170).
     if (P.inside && S.absorbing) lane_absorption(P, S, k_hat, hit.t);
     return BOUNCE_CONTINUE;
+}
+
+IX_DEV int bounce_hit(const Group& g, LanePath& P, const DevScene& S, const float4* __restrict__ planes, float& esc,
+                      float& t) {
+    return bounce_at(P, S, planes, group_next_hit(g, P, planes, (int)S.s.n_planes), esc, t);
 }
 
 IX_DEV void bounce_geometry(const LanePath& P, const DevScene& S, const float4* __restrict__ planes, float t,
@@ -1009,6 +1016,16 @@ IX_DEV int group_bounce(const Group& g, LanePath& P, const DevScene& S,
                         const float4* __restrict__ planes, float& esc) {
     float t = 0.0f;
     if (bounce_hit(g, P, S, planes, esc, t) == BOUNCE_ESCAPED) return BOUNCE_ESCAPED;
+    BounceGeom G;
+    bounce_geometry(P, S, planes, t, G);
+    return bounce_arm(g, P, S, planes, G);
+}
+
+// ... of a path whose next hit is known.
+IX_DEV int group_bounce_at(const Group& g, LanePath& P, const DevScene& S, const float4* __restrict__ planes, Hit hit,
+                           float& esc) {
+    float t = 0.0f;
+    if (bounce_at(P, S, planes, hit, esc, t) == BOUNCE_ESCAPED) return BOUNCE_ESCAPED;
     BounceGeom G;
     bounce_geometry(P, S, planes, t, G);
     return bounce_arm(g, P, S, planes, G);
