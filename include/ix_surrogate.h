@@ -46,6 +46,20 @@ int ix_mlp_bias_grad(uint32_t m, uint32_t n, const float* dz, float* db, void* s
 /* Adam step t (1-based) on f32 weights w with moments m, v; wb (bf16 copy) may be NULL. */
 int ix_mlp_adam(uint64_t count, float* w, void* wb, const float* g, float* m, float* v, float lr, float beta1,
                 float beta2, float eps, uint32_t t, void* stream);
+/* The same step of n tensors in one launch (per 16 of them). */
+typedef struct ix_mlp_adam_tensor {
+    uint64_t count;
+    float* w;
+    void* wb; /* bf16 copy, may be NULL */
+    const float* g;
+    float* m;
+    float* v;
+} ix_mlp_adam_tensor;
+int ix_mlp_adam_multi(uint32_t n, const ix_mlp_adam_tensor* tensors, float lr, float beta1, float beta2, float eps,
+                      uint32_t t, void* stream);
+/* out[r][c] = y[r][c] * scale[c] + shift[c], the product rounded before the sum. */
+int ix_mlp_scale_shift(uint32_t m, uint32_t n, const float* y, const float* scale, const float* shift, float* out,
+                       void* stream);
 /* xb = bf16(x). */
 int ix_mlp_to_bf16(uint64_t count, const float* x, void* xb, void* stream);
 

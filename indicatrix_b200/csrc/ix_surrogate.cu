@@ -5,10 +5,13 @@
 // parameters to tilt-resolved brilliance / fire / scintillation measured on the tracer's
 // renders (ix_design.h) and screens candidate designs before the tracer re-renders the
 // survivors.  No reference counterpart: the reference has no tracer-trained surrogate.
+#include <cmath>
 #include <cstdint>
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+
+#include "../../include/ix_surrogate.h"
 
 namespace ix {
 namespace mlp {
@@ -66,19 +69,38 @@ __global__ void __launch_bounds__(32 * BIAS_ROWS) bias_grad_kernel(int m, int n,
     cluster.sync();  // the ranks' shared memory outlives the read
 }
 
-// Adam on f32 master weights, with their bf16 copy refreshed (Kingma & Ba 2015).
-__global__ void adam_kernel(int64_t count, float* __restrict__ w, __nv_bfloat16* __restrict__ wb,
-                            const float* __restrict__ g, float* __restrict__ mom, float* __restrict__ vel, float lr,
-                            float beta1, float beta2, float eps, float bias1, float bias2) {
+// Adam on f32 master weights, with their bf16 copy refreshed (Kingma & Ba 2015), of up to
+// ADAM_TENSORS tensors: blockIdx.y is the tensor.  A network's tensors are small (at most
+// 256 x 256: 1.6 MB of traffic, 2 us), so launches bound the step, and one launch updates
+// them all: 8 tensors 42 -> 16 us on the host's clock.
+constexpr int ADAM_TENSORS = 16;
+struct AdamLaunch {
+    ix_mlp_adam_tensor t[ADAM_TENSORS];
+    float lr, beta1, beta2, eps, bias1, bias2;
+};
+__global__ void __launch_bounds__(256) adam_kernel(const __grid_constant__ AdamLaunch L) {
+    const ix_mlp_adam_tensor& T = L.t[blockIdx.y];
+    __nv_bfloat16* const wb = (__nv_bfloat16*)T.wb;
+    const int64_t count = (int64_t)T.count;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = beta1 * mom[i] + (1.0f - beta1) * gi;
-        const float vi = beta2 * vel[i] + (1.0f - beta2) * gi * gi;
-        mom[i] = mi;
-        vel[i] = vi;
-        const float wi = w[i] - lr * (mi / bias1) / (sqrtf(vi / bias2) + eps);
-        w[i] = wi;
+        const float gi = T.g[i];
+        const float mi = L.beta1 * T.m[i] + (1.0f - L.beta1) * gi;
+        const float vi = L.beta2 * T.v[i] + (1.0f - L.beta2) * gi * gi;
+        T.m[i] = mi;
+        T.v[i] = vi;
+        const float wi = T.w[i] - L.lr * (mi / L.bias1) / (sqrtf(vi / L.bias2) + L.eps);
+        T.w[i] = wi;
         if (wb) wb[i] = __float2bfloat16_rn(wi);
+    }
+}
+
+// The network's standardised outputs as metrics.
+__global__ void scale_shift_kernel(int64_t count, uint32_t n, const float* __restrict__ y,
+                                   const float* __restrict__ scale, const float* __restrict__ shift,
+                                   float* __restrict__ out) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t c = (uint32_t)(i % n);
+        out[i] = __fadd_rn(__fmul_rn(y[i], scale[c]), shift[c]);
     }
 }
 
@@ -116,10 +138,26 @@ cudaError_t bias_grad(int m, int n, const float* dz, float* db, cudaStream_t s) 
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, bias_grad_kernel, m, n, dz, db);
 }
-cudaError_t adam(int64_t count, float* w, void* wb, const float* g, float* mom, float* vel, float lr, float beta1,
-                 float beta2, float eps, float bias1, float bias2, cudaStream_t s) {
-    adam_kernel<<<grid_for(count), 256, 0, s>>>(count, w, (__nv_bfloat16*)wb, g, mom, vel, lr, beta1, beta2, eps,
-                                               bias1, bias2);
+cudaError_t adam(uint32_t n, const ix_mlp_adam_tensor* t, float lr, float beta1, float beta2, float eps, float bias1,
+                 float bias2, cudaStream_t s) {
+    for (uint32_t begin = 0; begin < n; begin += ADAM_TENSORS) {
+        const uint32_t k = n - begin < ADAM_TENSORS ? n - begin : ADAM_TENSORS;
+        AdamLaunch L{};
+        uint64_t most = 0;
+        for (uint32_t i = 0; i < k; ++i) {
+            L.t[i] = t[begin + i];
+            if (L.t[i].count > most) most = L.t[i].count;
+        }
+        L.lr = lr, L.beta1 = beta1, L.beta2 = beta2, L.eps = eps, L.bias1 = bias1, L.bias2 = bias2;
+        adam_kernel<<<dim3(grid_for((int64_t)most), k), 256, 0, s>>>(L);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+cudaError_t scale_shift(int64_t count, uint32_t n, const float* y, const float* scale, const float* shift, float* out,
+                        cudaStream_t s) {
+    scale_shift_kernel<<<grid_for(count), 256, 0, s>>>(count, n, y, scale, shift, out);
     return cudaGetLastError();
 }
 cudaError_t to_bf16(int64_t count, const float* x, void* xb, cudaStream_t s) {
@@ -129,10 +167,6 @@ cudaError_t to_bf16(int64_t count, const float* x, void* xb, cudaStream_t s) {
 
 }  // namespace mlp
 }  // namespace ix
-
-#include "../../include/ix_surrogate.h"
-
-#include <cmath>
 
 namespace {
 int rc(cudaError_t e) { return e == cudaSuccess ? 0 : 1; }
@@ -152,9 +186,22 @@ int ix_mlp_bias_grad(uint32_t m, uint32_t n, const float* dz, float* db, void* s
 }
 int ix_mlp_adam(uint64_t count, float* w, void* wb, const float* g, float* m, float* v, float lr, float beta1,
                 float beta2, float eps, uint32_t t, void* stream) {
-    if (!w || !g || !m || !v || t == 0) return 1;
+    const ix_mlp_adam_tensor one{count, w, wb, g, m, v};
+    return ix_mlp_adam_multi(1, &one, lr, beta1, beta2, eps, t, stream);
+}
+int ix_mlp_adam_multi(uint32_t n, const ix_mlp_adam_tensor* tensors, float lr, float beta1, float beta2, float eps,
+                      uint32_t t, void* stream) {
+    if (!tensors || t == 0) return 1;
+    for (uint32_t i = 0; i < n; ++i)
+        if (!tensors[i].w || !tensors[i].g || !tensors[i].m || !tensors[i].v) return 1;
     const float b1 = 1.0f - std::pow(beta1, (float)t), b2 = 1.0f - std::pow(beta2, (float)t);
-    return rc(ix::mlp::adam((int64_t)count, w, wb, g, m, v, lr, beta1, beta2, eps, b1, b2, st(stream)));
+    return rc(ix::mlp::adam(n, tensors, lr, beta1, beta2, eps, b1, b2, st(stream)));
+}
+int ix_mlp_scale_shift(uint32_t m, uint32_t n, const float* y, const float* scale, const float* shift, float* out,
+                       void* stream) {
+    if (m == 0 || n == 0) return 0;
+    if (!y || !scale || !shift || !out) return 1;
+    return rc(ix::mlp::scale_shift((int64_t)m * n, n, y, scale, shift, out, st(stream)));
 }
 int ix_mlp_to_bf16(uint64_t count, const float* x, void* xb, void* stream) {
     if (!x || !xb) return 1;
