@@ -18,8 +18,11 @@ namespace mlp {
 namespace {
 
 // Mean squared error over the m x n outputs: dy = 2 (y - t) / (m n) (f32 and bf16), and
-// the loss summed into *loss (one atomic per warp).
-__global__ void mse_grad_kernel(int m, int n, const float* __restrict__ y, const float* __restrict__ t,
+// the loss summed into *loss: a block's share in f64, then one f32 atomic.  The order of the
+// atomics is the scheduler's, so their number is what the loss's last bits depend on: 432 at
+// 4096 x 27, where one per warp made it 3456, all on one address (6.8 us; 2.5 us so).
+constexpr int MSE_THREADS = 256;
+__global__ void __launch_bounds__(MSE_THREADS) mse_grad_kernel(int m, int n, const float* __restrict__ y, const float* __restrict__ t,
                                 float* __restrict__ dy, __nv_bfloat16* __restrict__ dyb, float* __restrict__ loss) {
     const int64_t total = (int64_t)m * n;
     const float inv = 1.0f / (float)total;
@@ -31,8 +34,17 @@ __global__ void mse_grad_kernel(int m, int n, const float* __restrict__ y, const
         dyb[i] = __float2bfloat16_rn(g);
         part += d * d * inv;
     }
-    for (int off = 16; off > 0; off >>= 1) part += __shfl_down_sync(0xFFFFFFFFu, part, off);
-    if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, part);
+    if (!loss) return;
+    __shared__ double s_part[MSE_THREADS / 32];
+    double sum = (double)part;
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xFFFFFFFFu, sum, off);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double total_part = 0.0;
+        for (int i = 0; i < MSE_THREADS / 32; ++i) total_part += s_part[i];
+        atomicAdd(loss, (float)total_part);
+    }
 }
 
 // db[col] = sum over rows of dz.  Reading the rows bounds it (4 MB at 4096 x 256), so a
@@ -118,7 +130,7 @@ unsigned int grid_for(int64_t n) {
 
 cudaError_t mse_grad(int m, int n, const float* y, const float* t, float* dy, void* dyb, float* loss,
                      cudaStream_t s) {
-    mse_grad_kernel<<<grid_for((int64_t)m * n), 256, 0, s>>>(m, n, y, t, dy, (__nv_bfloat16*)dyb, loss);
+    mse_grad_kernel<<<grid_for((int64_t)m * n), MSE_THREADS, 0, s>>>(m, n, y, t, dy, (__nv_bfloat16*)dyb, loss);
     return cudaGetLastError();
 }
 cudaError_t bias_grad(int m, int n, const float* dz, float* db, cudaStream_t s) {

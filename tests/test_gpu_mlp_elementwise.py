@@ -77,3 +77,25 @@ def test_members_metrics_equal_numpy(m):
     ens.nets[2].t_mean = 0.5  # a plain number still broadcasts
     assert np.array_equal(ens.predict_members(x)[2], ens.nets[2].forward_device(xb)[0].cpu().numpy() *
                           ens.nets[2].t_std + 0.5)
+
+
+@pytest.mark.parametrize("m,n", [(1, 1), (255, 1), (256, 1), (257, 1), (4096, 27), (30000, 27)])
+def test_mse_loss_and_gradient_match_fp64(m, n):
+    import torch
+
+    from indicatrix_b200.surrogate import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    y, t = (torch.randn(m, n, device="cuda", generator=g) for _ in range(2))
+    dy, dyb = torch.empty_like(y), torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+    loss = torch.full((1,), 2.0, device="cuda")
+    assert _lib().ix_mlp_mse_grad(m, n, y.data_ptr(), t.data_ptr(), dy.data_ptr(), dyb.data_ptr(), loss.data_ptr(),
+                                  _stream()) == 0
+    d = y.double() - t.double()
+    eps = float(np.finfo(np.float32).eps)
+    want = 2.0 + float((d * d).mean())
+    # At most min(blocks, 2368) atomics, each half an ulp of a sum below 8, and 8 roundings a term.
+    blocks = min((m * n + 255) // 256, 148 * 16)
+    assert abs(float(loss) - want) <= (4 * blocks + 8 * (1 + m * n // (256 * blocks))) * eps + 8 * eps * want
+    assert bool(((dy.double() - 2 * d / (m * n)).abs() <= 4 * eps * (y.abs() + t.abs()).double() * 2 / (m * n)).all())
+    assert bool((dyb == dy.bfloat16()).all())
