@@ -15,8 +15,11 @@ namespace ix {
 // never count).  The second smallest is kept beside it: a winner ahead of it by two units
 // of 2^-16 relative -- the reciprocal, the product and the replaced bits err by less than
 // one -- is the plane the exact scan keeps, whatever the rounding.  Everything else (a
-// closer second, an origin on or outside a plane, no candidate, a winner the exact scan
-// would pass over) is undecided and takes the exact scan.
+// closer second, an origin on, outside or within 1e-20 of a plane, no candidate, a winner the
+// exact scan would pass over) is undecided and takes the exact scan.  The 1e-20 keeps every
+// key finite for normals up to 1e18: nearer than that the reciprocal overflows (a subnormal
+// side is flushed before it), and infinity with an index in its low bits is a NaN that the
+// minimum passes over.
 //
 // The planes come as pairs (i, i + 8) of a block of 16 in shared memory, lane c reading
 // pair c of each block, so that the packed f32x2 units form both planes' dot products:
@@ -115,7 +118,7 @@ IX_DEV bool warp_interior_hit(const float4* __restrict__ rows, const float4* __r
         u2 = fminf(fminf(u2, hi), fmaxf(u1, lo));
         u1 = fminf(u1, lo);
     }
-    u1 = most < 0.0f ? __uint_as_float(__float_as_uint(u1) | (uint32_t)c) : -INFINITY;
+    u1 = most < -1e-20f ? __uint_as_float(__float_as_uint(u1) | (uint32_t)c) : -INFINITY;
 #pragma unroll
     for (int m = 4; m > 0; m >>= 1) {
         const float o1 = __shfl_xor_sync(WARP_MASK, u1, m), o2 = __shfl_xor_sync(WARP_MASK, u2, m);
