@@ -134,12 +134,12 @@ cudaError_t mse_grad(int m, int n, const float* y, const float* t, float* dy, vo
     return cudaGetLastError();
 }
 cudaError_t bias_grad(int m, int n, const float* dz, float* db, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
+    if (n <= 0) return cudaErrorInvalidValue;  // no columns, or more than an int counts
     // One CTA does while the rows are one pass of it.
     int ranks = 1;
     while (ranks < BIAS_CLUSTER && (int64_t)ranks * BIAS_ROWS < m) ranks *= 2;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((n + 31) / 32) * (unsigned)ranks);
+    cfg.gridDim = dim3(((unsigned)n + 31u) / 32u * (unsigned)ranks);
     cfg.blockDim = dim3(32 * BIAS_ROWS);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -148,7 +148,8 @@ cudaError_t bias_grad(int m, int n, const float* dz, float* db, cudaStream_t s) 
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, bias_grad_kernel, m, n, dz, db);
+    (void)cudaLaunchKernelEx(&cfg, bias_grad_kernel, m, n, dz, db);
+    return cudaGetLastError();  // and leaves none for the next call to find
 }
 cudaError_t adam(uint32_t n, const ix_mlp_adam_tensor* t, float lr, float beta1, float beta2, float eps, float bias1,
                  float bias2, cudaStream_t s) {
