@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 
@@ -37,6 +38,7 @@ constexpr int THREADS = 256;      // 8 warps: staging and epilogue split over th
 constexpr int STAGES = 3;      // K slices in shared memory at once
 constexpr uint32_t WAIT_LIMIT = 1u << 24;  // mbarrier polls before a wait gives up
 constexpr int SM_COUNT = 148;
+constexpr int MAX_DEVICES = 64;
 
 enum Epilogue : int {
     EPI_STORE = 0,      // c = acc
@@ -398,16 +400,18 @@ __global__ void __launch_bounds__(256) split_sum_kernel(const float* __restrict_
 }
 
 template <int NT>
-cudaError_t launch_nt(const GemmParams& p, uint32_t splits, cudaStream_t st) {
+cudaError_t launch_nt(const GemmParams& p, uint32_t splits, int device, cudaStream_t st) {
     // The operand stages, reused by the epilogue's 8 warps x 32 x (NT / 2 + 1) f32 staging.
     constexpr int stage_bytes = STAGES * (TM + NT) * BK * 2, epi_bytes = (THREADS / 32) * 32 * (NT / 2 + 1) * 4;
     const int smem = stage_bytes > epi_bytes ? stage_bytes : epi_bytes;
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [&] {
-        attr = cudaFuncSetAttribute(umma_gemm_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    });
-    if (attr != cudaSuccess) return attr;
+    // The limit is an attribute of the kernel on the current device.
+    static std::atomic<bool> raised[MAX_DEVICES];
+    if (!raised[device].load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(umma_gemm_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+            cudaSuccess)
+            return cudaGetLastError();
+        raised[device].store(true, std::memory_order_release);
+    }
     const dim3 grid((p.m + TM - 1) / TM, (p.n + NT - 1) / NT, splits);
     umma_gemm_kernel<NT><<<grid, THREADS, smem, st>>>(p);
     return cudaGetLastError();
@@ -415,24 +419,32 @@ cudaError_t launch_nt(const GemmParams& p, uint32_t splits, cudaStream_t st) {
 
 __device__ unsigned int g_umma_status;
 
-// Split-K workspace (device, grown on demand; the surrogate's calls are not captured).
-std::mutex g_ws_mu;
-float* g_ws = nullptr;
-size_t g_ws_floats = 0;
+// Where the split-K partials live: each call takes its own stretch of a pool of its device, in
+// its stream's order, and gives it back behind its sum, so that calls on other streams or from
+// other threads never share one.  A call needs at most SM_COUNT tiles of 128 x 32 f32 (2.4 MB:
+// what splits has the narrowest tile); the pool holds on to KEEP_BYTES between calls at most
+// and returns the rest to the device at the next synchronisation.
+constexpr uint64_t KEEP_BYTES = 64ull << 20;
+std::mutex g_pools_mu;
+cudaMemPool_t g_pools[MAX_DEVICES];
 
-float* workspace(size_t floats) {
-    std::lock_guard<std::mutex> lk(g_ws_mu);
-    if (floats <= g_ws_floats) return g_ws;
-    if (g_ws) cudaFree(g_ws);
-    g_ws = nullptr;
-    g_ws_floats = 0;
-    if (cudaMalloc(&g_ws, floats * sizeof(float)) != cudaSuccess) {
-        (void)cudaGetLastError();
-        g_ws = nullptr;
-        return nullptr;
+cudaMemPool_t partials_pool(int device) {
+    std::lock_guard<std::mutex> lk(g_pools_mu);
+    cudaMemPool_t& pool = g_pools[device];
+    if (pool) return pool;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = KEEP_BYTES;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        pool = nullptr;
+    } else if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        (void)cudaMemPoolDestroy(pool);
+        pool = nullptr;
     }
-    g_ws_floats = floats;
-    return g_ws;
+    if (!pool) (void)cudaGetLastError();
+    return pool;
 }
 
 uint32_t tiles(uint32_t x, uint32_t t) { return (x + t - 1) / t; }
@@ -442,6 +454,11 @@ int run(GemmParams p, void* stream) {
     if (p.k == 0 || !p.a || !p.b) return 1;
     if (p.m > (1u << 30) || p.n > (1u << 30) || p.k > (1u << 30)) return 1;
     void* st_ptr = nullptr;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device >= MAX_DEVICES) {
+        (void)cudaGetLastError();
+        return 1;
+    }
     if (cudaGetSymbolAddress(&st_ptr, g_umma_status) != cudaSuccess) {
         (void)cudaGetLastError();
         return 1;
@@ -466,19 +483,25 @@ int run(GemmParams p, void* stream) {
     if (splits > 1) splits = tiles(p.k, p.k_split);  // every split non-empty
     float* c = p.out_f32;
     const uint32_t ldc = p.ldo;
+    float* partials = nullptr;
     if (splits > 1) {
-        float* ws = workspace((size_t)splits * p.m * p.n);
-        if (!ws) return 1;
-        p.out_f32 = ws;
+        const cudaMemPool_t pool = partials_pool(device);
+        if (!pool) return 1;
+        if (cudaMallocFromPoolAsync((void**)&partials, (size_t)splits * p.m * p.n * sizeof(float), pool, s) !=
+            cudaSuccess) {
+            (void)cudaGetLastError();
+            return 1;
+        }
+        p.out_f32 = partials;
         p.ldo = p.n;
         p.out_bf16 = nullptr;
     }
     cudaError_t e;
     switch (nt) {
-        case 32: e = launch_nt<32>(p, splits, s); break;
-        case 64: e = launch_nt<64>(p, splits, s); break;
-        case 128: e = launch_nt<128>(p, splits, s); break;
-        default: e = launch_nt<256>(p, splits, s); break;
+        case 32: e = launch_nt<32>(p, splits, device, s); break;
+        case 64: e = launch_nt<64>(p, splits, device, s); break;
+        case 128: e = launch_nt<128>(p, splits, device, s); break;
+        default: e = launch_nt<256>(p, splits, device, s); break;
     }
     if (e == cudaSuccess && splits > 1) {
         const uint64_t count = (uint64_t)p.m * p.n;
@@ -486,6 +509,10 @@ int run(GemmParams p, void* stream) {
         if (blocks > (uint64_t)SM_COUNT * 8) blocks = (uint64_t)SM_COUNT * 8;
         split_sum_kernel<<<(unsigned)blocks, 256, 0, s>>>(p.out_f32, splits, p.m, p.n, p.ldo, c, ldc);
         e = cudaGetLastError();
+    }
+    if (partials && cudaFreeAsync(partials, s) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 1;
     }
     return e == cudaSuccess ? 0 : 1;
 }
