@@ -1478,6 +1478,7 @@ int ix_evaluate_gem_optical_metrics_batch(ix_backend* b, const ix_metrics_stone*
     if (!exit_lighting_setup(*lighting, &L.env, &L.spec, &L.factor, &L.head_shadow_cos, L.dirs)) return IX_DECLINED;
     L.want_fire = want_fire_and_scintillation ? 1u : 0u;
     L.n_poses = n_poses;
+    L.sm_count = (uint32_t)b->sm_count;
     std::vector<float> planes;
     std::vector<ix::MetricsStoneDev> dstones(n_stones);
     std::vector<double> wplanes;

@@ -277,6 +277,7 @@ struct MetricsLaunch {
     const ExtentsDev* extents;      // device, per stone (the girdle half-width, fan.rs:34)
     const MetricsPoseDev* poses;    // device
     uint32_t n_poses;
+    uint32_t sm_count;              // the device's, for the warps a pose gets
     uint32_t want_fire;             // fire and scintillation rays traced
     ix_environment env;             // the scoring light: exposure 1, no tray, default shadow
     float spec;                     // its spectral power at 550 nm

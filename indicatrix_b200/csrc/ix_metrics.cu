@@ -482,9 +482,9 @@ cudaError_t IX_SFX(launch_metrics)(const MetricsLaunch& l, cudaStream_t stream) 
     if (l.n_poses == 0) return cudaSuccess;
     // Warps a pose gets: 16 per SM shared among the poses, 4 to 16 of a CTA, then CTAs of a
     // cluster.
-    constexpr uint32_t TARGET_WARPS = 148 * 16;
+    const uint64_t target_warps = (uint64_t)l.sm_count * 16;
     uint32_t warps = 4;
-    while (warps < MAX_WARPS * MAX_CLUSTER && (uint64_t)2 * warps * l.n_poses <= TARGET_WARPS) warps *= 2;
+    while (warps < MAX_WARPS * MAX_CLUSTER && (uint64_t)2 * warps * l.n_poses <= target_warps) warps *= 2;
     const uint32_t ranks = warps > MAX_WARPS ? warps / MAX_WARPS : 1u;
     const uint32_t threads = (warps / ranks) * 32u, groups = threads / 8u;
     const uint32_t total = (l.want_fire ? 2u : 1u) * MAX_RAYS;
