@@ -54,6 +54,7 @@ __global__ void __launch_bounds__(MSE_THREADS) mse_grad_kernel(int m, int n, con
 // thread per column walking the rows, 7.5 us so.
 constexpr int BIAS_ROWS = 32;     // rows of a CTA pass
 constexpr int BIAS_CLUSTER = 8;
+constexpr int BIAS_WARPS = 4;     // of the wide kernel's CTA
 __global__ void __launch_bounds__(32 * BIAS_ROWS) bias_grad_kernel(int m, int n, const float* __restrict__ dz,
                                                                   float* __restrict__ db) {
     namespace cg = cooperative_groups;
@@ -79,6 +80,58 @@ __global__ void __launch_bounds__(32 * BIAS_ROWS) bias_grad_kernel(int m, int n,
         db[col] = total;
     }
     cluster.sync();  // the ranks' shared memory outlives the read
+}
+
+// The same sums, in the same order, by one CTA of 4 warps for 32 columns: warp y takes rows y,
+// y + 4, ... of a pass, whose partial sums fold in the thread that holds them, and the ranks
+// follow one another.  For few rows, where a cluster's barriers are most of its time, and for
+// columns enough to fill the GPU without splitting their rows, where 1024-thread CTAs cost
+// a wave each (us, clusters / so / a thread per column): 64 x 256 4.8 / 3.9 / 4.0, 33 x 100000
+// 68 / 8.3 / 4.3, 1000 x 20000 73 / 14 / 27.  With 2 and 8 warps 64 x 256 takes 8.3 and 4.1,
+// 1024 x 16384 74 and 14.4 against 12.4.
+__global__ void __launch_bounds__(32 * BIAS_WARPS) bias_grad_wide_kernel(int m, int n, int ranks,
+                                                                        const float* __restrict__ dz,
+                                                                        float* __restrict__ db) {
+    constexpr int WARPS = BIAS_WARPS, ROWS = BIAS_ROWS / WARPS;  // rows of a pass in one thread
+    __shared__ float s_part[BIAS_CLUSTER][WARPS][32];
+    const int c = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int64_t col = blockIdx.x * (int64_t)32 + c, row = (int64_t)WARPS * n, step = (int64_t)ranks * BIAS_ROWS;
+    for (int rank = 0; rank < ranks; ++rank) {
+        float v[ROWS];
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) v[i] = 0.0f;
+        if (col < n) {
+            int64_t r = (int64_t)rank * BIAS_ROWS + y;
+            const float* p = dz + r * n + col;
+            for (; r + (ROWS - 1) * WARPS < m; r += step, p += step * n) {
+#pragma unroll
+                for (int i = 0; i < ROWS; ++i) v[i] += p[i * row];
+            }
+#pragma unroll
+            for (int i = 0; i < ROWS - 1; ++i)
+                if (r + i * WARPS < m) v[i] += p[i * row];
+        }
+#pragma unroll
+        for (int off = ROWS / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int i = 0; i < off; ++i) v[i] += v[i + off];
+        s_part[rank][y][c] = v[0];
+    }
+    __syncthreads();
+    if (y == 0 && col < n) {
+        float total = 0.0f;
+        for (int k = 0; k < ranks; ++k) {
+            float v[WARPS];
+#pragma unroll
+            for (int i = 0; i < WARPS; ++i) v[i] = s_part[k][i][c];
+#pragma unroll
+            for (int off = WARPS / 2; off > 0; off >>= 1)
+#pragma unroll
+                for (int i = 0; i < off; ++i) v[i] += v[i + off];
+            total += v[0];
+        }
+        db[col] = total;
+    }
 }
 
 // Adam on f32 master weights, with their bf16 copy refreshed (Kingma & Ba 2015), of up to
@@ -138,8 +191,15 @@ cudaError_t bias_grad(int m, int n, const float* dz, float* db, cudaStream_t s) 
     // One CTA does while the rows are one pass of it.
     int ranks = 1;
     while (ranks < BIAS_CLUSTER && (int64_t)ranks * BIAS_ROWS < m) ranks *= 2;
+    // Clusters pay up to a wave of their CTAs (two an SM: 5 us, 12 ns for each CTA past it); the
+    // wide kernel pays 3 us and 7 ns a row.  Either gives the same bits.
+    const int64_t groups = ((int64_t)n + 31) / 32, ctas = groups * ranks, wave = 2 * 148;
+    if (m <= 128 + 2 * (ctas > wave ? ctas - wave : 0)) {
+        bias_grad_wide_kernel<<<(unsigned)groups, 32 * BIAS_WARPS, 0, s>>>(m, n, ranks, dz, db);
+        return cudaGetLastError();
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(((unsigned)n + 31u) / 32u * (unsigned)ranks);
+    cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(32 * BIAS_ROWS);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
