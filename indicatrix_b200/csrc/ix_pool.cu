@@ -111,12 +111,14 @@ IX_DEV uint32_t pool_loop(const Group& g, uint32_t* counter, uint32_t total_chun
     bool busy = false;  // the group has a path in flight (group-uniform)
     uint32_t row = 0;   // ... and its accumulator row
     uint32_t drops = 0;
-    // A group that has had no path yet takes part in the warp's scan and colour sum, its
-    // result unused: what those read of it is set here.
     LanePath P;
-    P.o = P.d = v3(0.0f, 0.0f, 0.0f);
-    P.lambda = P.pdf = P.split = 0.0f;
-    P.compat = 0u;
+    if constexpr (UNI == TRANSPORT_ISOTROPIC) {
+        // A group that has had no path yet takes part in the warp's scan and colour sum, its
+        // result unused: what those read of it is set here.
+        P.o = P.d = v3(0.0f, 0.0f, 0.0f);
+        P.lambda = P.pdf = P.split = 0.0f;
+        P.compat = 0u;
+    }
     for (;;) {
         const unsigned idle = __ballot_sync(FULL, !busy) & 0x01010101u;
         const uint32_t n_idle = __popc(idle);
