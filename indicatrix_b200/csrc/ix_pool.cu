@@ -98,6 +98,13 @@ IX_DEV uint32_t pool_fill(WarpPool& wp, const PoolJob& J, uint32_t chunk, uint32
 // with the warp converged and its groups idle).  The k-th claim on `counter` takes chunk
 // k * stride while that is below total_chunks; a chunk is `size` paths, at most POOL_CHUNK.
 // Returns the samples this lane dropped.
+//
+// The fast build's isotropic loop scans and sums colours with the warp converged: shuffles
+// under each group's own mask repeat per group, and the loop stalls on instruction fetch (74 -> 66
+// KB, 256 x 256 x 64 9.20 -> 8.74 ms).  The exact build ran slower so (16.0 -> 17.4 ms, a batch
+// 20.1 -> 20.7), so there each group scans for itself.  The sums are the same.
+template <int UNI>
+constexpr bool CONVERGED = UNI == TRANSPORT_ISOTROPIC && !IX_EXACT;
 template <int UNI, class JobOf, class LoadPlanes>
 IX_DEV uint32_t pool_loop(const Group& g, uint32_t* counter, uint32_t total_chunks, uint32_t size, uint32_t stride,
                           WarpPool& wp, JobOf job_of, LoadPlanes load_planes) {
@@ -112,7 +119,7 @@ IX_DEV uint32_t pool_loop(const Group& g, uint32_t* counter, uint32_t total_chun
     uint32_t row = 0;   // ... and its accumulator row
     uint32_t drops = 0;
     LanePath P;
-    if constexpr (UNI == TRANSPORT_ISOTROPIC) {
+    if constexpr (CONVERGED<UNI>) {
         // A group that has had no path yet takes part in the warp's scan and colour sum, its
         // result unused: what those read of it is set here.
         P.o = P.d = v3(0.0f, 0.0f, 0.0f);
@@ -165,7 +172,7 @@ IX_DEV uint32_t pool_loop(const Group& g, uint32_t* counter, uint32_t total_chun
         }
         head += min(n_idle, avail);
         const PoolJob& J = wp.job;
-        if constexpr (UNI == TRANSPORT_ISOTROPIC) {
+        if constexpr (CONVERGED<UNI>) {
             if (n_idle == 4 && avail == 0) continue;  // no path, and no job's planes yet
             const DevScene S = make_scene(*J.scene, J.flags);
             if (fresh) {
