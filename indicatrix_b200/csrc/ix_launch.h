@@ -245,7 +245,7 @@ struct CheckLaunch {
     uint32_t* out;        // device
 };
 
-// Analytic optical metrics (ix_metrics.cu): one CTA per pose.
+// Analytic optical metrics (ix_metrics.cu): a cluster of 1 to 8 CTAs per pose.
 struct MetricsStoneDev {
     uint32_t plane_offset;  // first float4 of the stone in `planes`
     uint32_t n_planes;

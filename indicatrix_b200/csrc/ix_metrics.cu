@@ -5,7 +5,8 @@
 // (classify.rs) -- a single-index interior trace of at most 10 bounces
 // (ray_trace.rs:264-352), with n_F / n_C companion traces for fire -- and 5 yaw-jittered
 // rays for temporal scintillation (scintillation.rs:85): 900 or 1800 independent rays.
-// What bounds them is latency: a ray is up to 33 scans of the planes, one after another.
+// What bounds them is latency: a ray is up to 31 scans of the planes, one after another (its
+// entry, then 10 bounces at each of three wavelengths).
 // So a ray is traced by 8 lanes that share each scan (ix_interior.cuh), four rays to a
 // warp, and the rays of a pose are spread over as many warps as the launch leaves it: 4
 // warps of one CTA when the poses fill the GPU, up to a cluster of 8 CTAs x 16 warps for one

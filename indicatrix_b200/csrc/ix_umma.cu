@@ -121,9 +121,10 @@ __device__ __forceinline__ float silu_grad(float z) {
 // The transposed view of an operand (rows adjacent in memory, 16-byte aligned columns, every
 // row of the tile and k of the slice inside the matrix): a thread reads 8 rows of two
 // neighbouring k and writes eight 4-byte pairs.  The pairs of 8 threads with neighbouring
-// row octets fall on the same four banks, so each thread starts at another of its eight rows
-// and the warp's stores never conflict.  Memory latency bounds it, so a thread issues every
-// load of the slice before its first store.  The weight gradient 256 x 256 x 4096 took 46 us with
+// row octets fall on the same four banks, so each thread starts at another of its eight rows:
+// no conflicts at R = 64, two ways at 32 and 128 (octets o and o + 8 of a warp share a bank),
+// four at 256.  Memory latency bounds it, so a thread issues every load of the slice before its
+// first store.  The weight gradient 256 x 256 x 4096 took 46 us with
 // 2-byte loads and stores, 16.7 us with a load and a store in turn, 14.6 us so.
 template <int R>
 __device__ void stage_turned(uint8_t* stage, const __nv_bfloat16* g, int64_t ks, uint32_t r0, uint32_t k0) {
@@ -303,9 +304,10 @@ __global__ void __launch_bounds__(THREADS) umma_gemm_kernel(const __grid_constan
         // Epilogue: warp w reads TMEM lane quadrant w % 4 (tile rows 32 (w % 4) ..) and
         // column half w / 4; each tcgen05.ld gives a thread 8 consecutive columns of its
         // row.  The warp's 32 x NT/2 block goes through shared memory (the operand stages
-        // are free now; rows padded by one word, so both passes are conflict-free) and
-        // leaves row by row with the lanes on consecutive columns: every store and every
-        // z_prev / bias load is coalesced.
+        // are free now; rows padded by one word, so the first pass has no conflicts) and
+        // leaves row by row with the lanes on consecutive columns, or four columns a lane (two-
+        // way conflicts at NT 32 and 128, four-way at 256): every store and every z_prev /
+        // bias load is coalesced.
         constexpr int HW = NT / 2;
         const uint32_t quad = warp & 3u, half = warp >> 2;
         float* stage = reinterpret_cast<float*>(smem) + warp * 32 * (HW + 1);
