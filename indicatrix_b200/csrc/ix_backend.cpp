@@ -196,6 +196,7 @@ int accumulate_impl(ix_backend* b, const ix_scene* scene, uint32_t sample_offset
     if (n_pixels == 0 || spp == 0) return IX_DONE;
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
+    if (fail(b, order_enter(b->trace_order, b->stream), "stream order")) return IX_DECLINED;
     if (fail(b, grow_device(&b->d_planes, &b->planes_cap, (size_t)scene->n_planes * 4), "planes alloc"))
         return IX_DECLINED;
     if (fail(b, grow_device(&b->d_sums, &b->sums_cap, (size_t)n_pixels * 3), "sums alloc"))
@@ -478,6 +479,7 @@ void ix_backend_destroy(ix_backend* b) {
     if (b->h_sums) cudaFreeHost(b->h_sums);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
+    order_free(b->trace_order);
     if (b->stream) cudaStreamDestroy(b->stream);
     (void)cudaGetLastError();
     delete b;
@@ -619,7 +621,8 @@ int ix_accumulate_attributed(ix_backend* b, const ix_scene* scene, const ix_metr
     const size_t records = (size_t)std::min<uint64_t>(n_pixels * spp, std::max<uint64_t>(max_budget, spp));
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
-    if (fail(b, grow_device(&b->d_planes, &b->planes_cap, (size_t)scene->n_planes * 4), "planes alloc") ||
+    if (fail(b, order_enter(b->trace_order, b->stream), "stream order") ||
+        fail(b, grow_device(&b->d_planes, &b->planes_cap, (size_t)scene->n_planes * 4), "planes alloc") ||
         fail(b, grow_device(&b->d_sums, &b->sums_cap, (size_t)n_pixels * 3), "sums alloc") ||
         fail(b, grow_pinned(&b->h_sums, &b->hsums_cap, (size_t)n_pixels * 3), "host alloc") ||
         fail(b, grow_device(&b->d_attr_cls, &b->attr_cls_cap, records), "attribution alloc") ||
@@ -695,6 +698,7 @@ struct ix_batch_plan {
     double* d_out = nullptr;
     uint32_t* d_counter = nullptr;
     unsigned long long* d_dropped = nullptr;
+    StreamOrder order;  // of the plan's buffers
     std::vector<ix::BatchJob> jobs;
     std::vector<uint64_t> job_out;  // first double of each job's sums
     std::vector<uint32_t> h_max_bounces;  // per scene
@@ -876,11 +880,13 @@ cudaError_t plan_enqueue(ix_batch_plan* p, cudaStream_t st, uint32_t variant, ui
 int plan_run_locked(ix_batch_plan* p, cudaStream_t st) {
     ix_backend* b = p->b;
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
+    if (fail(b, order_enter(p->order, st), "stream order")) return IX_DECLINED;
     if (p->variant == (uint32_t)ix::VARIANT_WAVEFRONT) {
         // Host-driven: its iteration count depends on the paths, so it is not one graph.
         if (fail(b, cudaEventRecord(b->ev0, st), "event")) return IX_DECLINED;
         if (fail(b, plan_run_wavefront(p, st), "wavefront")) return IX_DECLINED;
         if (fail(b, cudaEventRecord(b->ev1, st), "event")) return IX_DECLINED;
+        if (fail(b, order_leave(p->order, st), "stream order")) return IX_DECLINED;
         b->timing.paths = p->paths;
         b->timing.launches = 3 * p->wf_iterations + 2;
         return IX_DONE;
@@ -898,12 +904,14 @@ int plan_run_locked(ix_batch_plan* p, cudaStream_t st) {
     if (fail(b, cudaEventRecord(b->ev0, st), "event")) return IX_DECLINED;
     if (fail(b, cudaGraphLaunch(p->exec, st), "graph launch")) return IX_DECLINED;
     if (fail(b, cudaEventRecord(b->ev1, st), "event")) return IX_DECLINED;
+    if (fail(b, order_leave(p->order, st), "stream order")) return IX_DECLINED;
     b->timing.paths = p->paths;
     b->timing.launches = ix::shape_is_pool(ix::variant_shape((int)p->variant)) ? 2 : 1;
     return IX_DONE;
 }
 int plan_download_locked(ix_batch_plan* p, double* host_out) {
     ix_backend* b = p->b;
+    if (fail(b, order_enter(p->order, b->stream), "stream order")) return -1;
     if (fail(b, cudaMemcpyAsync(host_out, p->d_out, p->out_doubles * sizeof(double), cudaMemcpyDeviceToHost,
                                 b->stream), "batch download"))
         return -1;
@@ -1060,6 +1068,7 @@ int ix_batch_plan_autotune(ix_batch_plan* p, int reps, uint32_t* chosen) {
     ix_backend* b = p->b;
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return -1;
+    if (fail(b, order_enter(p->order, b->stream), "stream order")) return -1;
     // Each candidate is timed on every stride-th task / chunk of the plan: about 1/16 of
     // its work, spread over all its jobs, and never fewer claims than the grid has warps.
     // The sample ranks the candidates; the best kFinalists then run the whole plan once
@@ -1173,6 +1182,7 @@ void ix_batch_plan_destroy(ix_batch_plan* p) {
     cudaFree(p->wf_counts);
     cudaFree(p->wf_claim);
     if (p->h_wf) cudaFreeHost(p->h_wf);
+    order_free(p->order);
     (void)cudaGetLastError();
     delete p;
 }
@@ -1291,10 +1301,12 @@ int ix_accumulate_device(ix_backend* b, const ix_scene* scene, uint32_t sample_o
     cudaStream_t st = stream ? (cudaStream_t)stream : b->stream;
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     bool cancelled = false;
+    if (fail(b, order_enter(b->trace_order, st), "stream order")) return IX_DECLINED;
     if (fail(b, cudaEventRecord(b->ev0, st), "event")) return IX_DECLINED;
     int launches = enqueue_frame(b, *scene, sample_offset, spp, d_accum_xyz, accumulate, st, nullptr, &cancelled);
     if (launches < 0) return IX_DECLINED;
     if (fail(b, cudaEventRecord(b->ev1, st), "event")) return IX_DECLINED;
+    if (fail(b, order_leave(b->trace_order, st), "stream order")) return IX_DECLINED;
     b->timing.paths = (uint64_t)scene->width * scene->height * spp;
     b->timing.launches = (uint32_t)launches * kernels_per_launch(b, *scene);
     return IX_DONE;

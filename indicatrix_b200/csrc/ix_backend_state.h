@@ -13,6 +13,14 @@
 #include <mutex>
 #include <string>
 
+// Device buffers that calls on several streams share: a call on another stream than the last
+// one that was left in flight waits for that on the device (order_enter, order_leave).
+struct StreamOrder {
+    cudaEvent_t done = nullptr;  // behind the last call left in flight
+    bool in_flight = false;
+    unsigned long long stream = 0;  // the id of that call's stream: a handle may name another later
+};
+
 struct DisplayState;  // the display pipeline's pooled buffers (ix_display_host.cpp)
 void display_state_free(DisplayState* d);
 struct RadianceState;  // the radiance codec's device and pinned buffers (ix_radiance.cpp)
@@ -59,6 +67,8 @@ struct ix_backend {
     // Fixed-point per-pixel sums of the path-pool kernels (FIXED_WORDS per pixel of a launch).
     unsigned long long* d_acc = nullptr;
     size_t acc_cap = 0;
+    // Of the single-scene calls' counters and sums above.
+    StreamOrder trace_order;
     // The metrics call's stones, poses and results.
     uint8_t* d_metrics = nullptr;
     size_t metrics_cap = 0;
@@ -115,6 +125,33 @@ inline bool fail(ix_backend* b, cudaError_t e, const char* where) {
     b->last_error = std::string(where) + ": " + cudaGetErrorString(e);
     (void)cudaGetLastError();
     return true;
+}
+
+inline bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) != cudaSuccess) (void)cudaGetLastError();
+    return s != cudaStreamCaptureStatusNone;
+}
+// A captured call runs when its graph does, which only the caller can order; a wait for work
+// outside of the capture would end it.
+inline cudaError_t order_enter(const StreamOrder& o, cudaStream_t st) {
+    if (!o.in_flight || capturing(st)) return cudaSuccess;
+    unsigned long long id = 0;
+    const cudaError_t e = cudaStreamGetId(st, &id);  // not permitted under capture
+    if (e != cudaSuccess || id == o.stream) return e;
+    return cudaStreamWaitEvent(st, o.done, 0);
+}
+// After a call that returns before its work on `st` is done.
+inline cudaError_t order_leave(StreamOrder& o, cudaStream_t st) {
+    if (capturing(st)) return cudaSuccess;
+    cudaError_t e = o.done ? cudaSuccess : cudaEventCreateWithFlags(&o.done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamGetId(st, &o.stream);
+    if (e == cudaSuccess) e = cudaEventRecord(o.done, st);
+    if (e == cudaSuccess) o.in_flight = true;
+    return e;
+}
+inline void order_free(StreamOrder& o) {
+    if (o.done) cudaEventDestroy(o.done);
 }
 
 template <typename T>

@@ -122,6 +122,7 @@ struct DisplayState {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     ix_display_timing timing{0.0f, 0.0f, 0.0f, 0, 0};
     bool pending = false;  // an asynchronous call's events are still to be read
+    StreamOrder order;     // of the buffers above
 };
 
 void display_state_free(DisplayState* d) {
@@ -142,6 +143,7 @@ void display_state_free(DisplayState* d) {
     cudaFree(d->d_rgba);
     for (cudaEvent_t e : d->ev)
         if (e) cudaEventDestroy(e);
+    order_free(d->order);
     delete d;
 }
 
@@ -406,7 +408,8 @@ int ix_generate_guide_buffers(ix_backend* b, uint32_t width, uint32_t height, co
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     DisplayState* d = state(b);
-    cudaError_t e = grow_device(&d->d_planes, &d->planes_cap, 4 * (size_t)std::max(n_planes, 1u));
+    cudaError_t e = order_enter(d->order, b->stream);
+    if (e == cudaSuccess) e = grow_device(&d->d_planes, &d->planes_cap, 4 * (size_t)std::max(n_planes, 1u));
     if (e == cudaSuccess) e = grow_device(&d->d_depth, &d->depth_cap, n);
     if (e == cudaSuccess) e = grow_device(&d->d_normal, &d->normal_cap, 3 * n);
     if (e == cudaSuccess) e = grow_device(&d->d_facet, &d->facet_cap, n);
@@ -448,6 +451,7 @@ int ix_atrous_denoise(ix_backend* b, const float* color, const float* depth, con
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     DisplayState* d = state(b);
+    if (fail(b, order_enter(d->order, b->stream), "stream order")) return IX_DECLINED;
     if (!alloc_frame(b, d, n, true, true, false)) return IX_DECLINED;
     d->cached = false;
     const auto t0 = std::chrono::steady_clock::now();
@@ -487,7 +491,8 @@ static int tonemap_impl(ix_backend* b, const float* xyz, uint64_t pixels, float 
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     DisplayState* d = state(b);
-    cudaError_t e = grow_device(&d->d_xyz, &d->xyz_cap, 3 * pixels);
+    cudaError_t e = order_enter(d->order, b->stream);
+    if (e == cudaSuccess) e = grow_device(&d->d_xyz, &d->xyz_cap, 3 * pixels);
     if (e == cudaSuccess) e = grow_device(&d->d_rgba, &d->rgba_cap, pixels);
     if (fail(b, e, "tonemap buffers")) return IX_DECLINED;
     const auto t0 = std::chrono::steady_clock::now();
@@ -536,6 +541,7 @@ int ix_denoise_and_tonemap_frame(ix_backend* b, uint32_t width, uint32_t height,
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     DisplayState* d = state(b);
+    if (fail(b, order_enter(d->order, b->stream), "stream order")) return IX_DECLINED;
     if (!alloc_frame(b, d, n, true, true, true)) return IX_DECLINED;
     d->cached = false;
     const auto t0 = std::chrono::steady_clock::now();
@@ -587,6 +593,7 @@ static int display_frame_impl(ix_backend* b, const ix_scene* scene, uint32_t wit
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     const cudaStream_t st = stream ? stream : b->stream;
     DisplayState* d = state(b);
+    if (fail(b, order_enter(d->order, st), "stream order")) return IX_DECLINED;
     if (!alloc_frame(b, d, n, false, accum_dev == nullptr, rgba_dev == nullptr)) return IX_DECLINED;
     if (fail(b, grow_device(&d->d_planes, &d->planes_cap, 4 * (size_t)std::max(sc.n_planes, 1u)), "planes"))
         return IX_DECLINED;
@@ -633,6 +640,7 @@ static int display_frame_impl(ix_backend* b, const ix_scene* scene, uint32_t wit
     }
     record(d, 3, st);
     // The host form waits for its RGBA8; the device form stays asynchronous on `st`.
+    if (!rgba_host && e == cudaSuccess) e = order_leave(d->order, st);
     if (rgba_host && e == cudaSuccess) e = d2h_staged(d, rgba_host, d->d_rgba, 4 * n, st);
     if (fail(b, e, "display frame")) {
         d->cached = false;
