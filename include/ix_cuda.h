@@ -187,7 +187,8 @@ void ix_batch_plan_destroy(ix_batch_plan* p);
  * pointers (IX_DECLINED for one that is not device or managed memory; the tools are
  * counted but not read on the host, so the caller validates them with ix_tool_validate);
  * the launch is enqueued on `stream` (a cudaStream_t, or NULL for the backend's own
- * stream) and not synchronised.
+ * stream) and not synchronised; calls on several streams run one after another (they share
+ * the backend's counters).
  * `accumulate` = 1 adds into d_accum_xyz, 0 overwrites it. */
 int ix_accumulate_device(ix_backend* b, const ix_scene* scene, uint32_t sample_offset,
                          uint32_t spp, double* d_accum_xyz, int accumulate, void* stream);

@@ -114,7 +114,8 @@ int ix_display_frame(struct ix_backend* b, const ix_scene* scene, uint32_t with_
 /* Device-resident form of ix_display_frame (no counterpart in the reference): `accum` and
  * `rgba` are device pointers, scene->planes stays a host pointer (it keys the guide
  * cache); the kernels are enqueued on `stream` (a cudaStream_t, NULL for the backend's
- * own) and not synchronised.  With spp == 0 the frame is opaque black. */
+ * own) and not synchronised; calls on several streams share the guides in order and their
+ * passes overlap.  With spp == 0 the frame is opaque black. */
 int ix_display_frame_device(struct ix_backend* b, const ix_scene* scene, uint32_t with_signature,
                             uint32_t spp, const float* accum, const ix_atrous_params* params,
                             uint8_t* rgba, void* stream);

@@ -150,6 +150,16 @@ inline cudaError_t order_leave(StreamOrder& o, cudaStream_t st) {
     if (e == cudaSuccess) o.in_flight = true;
     return e;
 }
+// Whether the last call left in flight has ended (another thread's capture must not end by it).
+inline bool order_idle(StreamOrder& o) {
+    if (!o.in_flight) return true;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaEventQuery(o.done) == cudaSuccess) o.in_flight = false;
+    else (void)cudaGetLastError();  // not ready; an error proper shows at the next call
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    return !o.in_flight;
+}
 inline void order_free(StreamOrder& o) {
     if (o.done) cudaEventDestroy(o.done);
 }

@@ -86,6 +86,18 @@ private:
 
 constexpr size_t STAGE_CHUNK = 4u << 20;  // bytes per pinned slot
 
+// A frame's passes fill the GPU only in part (each one ends in a tail that the next waits
+// for), so frames on several streams gain from running side by side: in turn on three
+// streams 1920 x 1080 takes 170 us a frame and 300 x 200 29, with one set of buffers handed on
+// 200 and 65 (one stream: 199 and 63).  2 and 3 sets: 171 and 172, 37 and 32.
+constexpr int COLOUR_SLOTS = 4;
+struct ColourSlot {
+    float4* d_col[2] = {nullptr, nullptr};
+    size_t cap[2] = {0, 0};
+    StreamOrder order;
+    uint64_t turn = 0;  // of the last call that took it
+};
+
 struct DisplayState {
     // Pinned two-slot ring for host <-> device copies of caller buffers, and the threads
     // that fill and drain it.
@@ -103,13 +115,15 @@ struct DisplayState {
     size_t facet_cap = 0;
     uint32_t* d_sig = nullptr;
     size_t sig_cap = 0;
-    // Packed guides and the colour ping-pong of the passes.
+    // Packed guides: written by one call at a time, read by the frames of every stream.
     float4* d_nrm = nullptr;
     size_t nrm_cap = 0;
     int2* d_fs = nullptr;
     size_t fs_cap = 0;
-    float4* d_col[2] = {nullptr, nullptr};
-    size_t col_cap[2] = {0, 0};
+    StreamOrder guides;
+    // The colour ping-pong of the passes, one for each stream in flight.
+    ColourSlot slots[COLOUR_SLOTS];
+    uint64_t turns = 0;
     // Host-layout colour in / out (3 floats per pixel) and RGBA8 out.
     float* d_xyz = nullptr;
     size_t xyz_cap = 0;
@@ -122,7 +136,6 @@ struct DisplayState {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     ix_display_timing timing{0.0f, 0.0f, 0.0f, 0, 0};
     bool pending = false;  // an asynchronous call's events are still to be read
-    StreamOrder order;     // of the buffers above
 };
 
 void display_state_free(DisplayState* d) {
@@ -137,13 +150,16 @@ void display_state_free(DisplayState* d) {
     cudaFree(d->d_sig);
     cudaFree(d->d_nrm);
     cudaFree(d->d_fs);
-    cudaFree(d->d_col[0]);
-    cudaFree(d->d_col[1]);
+    for (ColourSlot& c : d->slots) {
+        cudaFree(c.d_col[0]);
+        cudaFree(c.d_col[1]);
+        order_free(c.order);
+    }
     cudaFree(d->d_xyz);
     cudaFree(d->d_rgba);
     for (cudaEvent_t e : d->ev)
         if (e) cudaEventDestroy(e);
-    order_free(d->order);
+    order_free(d->guides);
     delete d;
 }
 
@@ -212,11 +228,55 @@ Resolved resolve(const ix_atrous_params& p, uint32_t spp) {
     return r;
 }
 
-bool alloc_frame(ix_backend* b, DisplayState* d, uint64_t n, bool guides_raw, bool xyz, bool rgba) {
+// The call on `st` waits for every call left in flight on another stream.
+cudaError_t order_all(DisplayState* d, cudaStream_t st) {
+    cudaError_t e = order_enter(d->guides, st);
+    for (const ColourSlot& c : d->slots)
+        if (e == cudaSuccess) e = order_enter(c.order, st);
+    return e;
+}
+bool fits(const ColourSlot& c, uint64_t n) { return std::min(c.cap[0], c.cap[1]) >= n; }
+cudaError_t grow_slot(ColourSlot& c, uint64_t n) {
+    const cudaError_t e = grow_device(&c.d_col[0], &c.cap[0], n);
+    return e == cudaSuccess ? grow_device(&c.d_col[1], &c.cap[1], n) : e;
+}
+// The colour buffers for a frame of n pixels on `st`: those its stream used last, else some
+// that no call in flight uses, else the oldest call's, which `st` then waits for (also where
+// there is no memory for another set).  A captured frame takes a set that is large enough.
+cudaError_t take_slot(DisplayState* d, uint64_t n, cudaStream_t st, ColourSlot** out) {
+    ColourSlot* pick = nullptr;
+    if (capturing(st)) {
+        for (ColourSlot& c : d->slots)
+            if (!pick && fits(c, n)) pick = &c;
+        *out = pick ? pick : &d->slots[0];
+        return cudaSuccess;
+    }
+    unsigned long long id = 0;
+    const cudaError_t e = cudaStreamGetId(st, &id);
+    if (e != cudaSuccess) return e;
+    for (ColourSlot& c : d->slots)
+        if (!pick && c.order.in_flight && c.order.stream == id) pick = &c;
+    for (ColourSlot& c : d->slots)
+        if (!pick && order_idle(c.order)) pick = &c;
+    if (!pick || !fits(*pick, n)) {
+        ColourSlot* oldest = nullptr;
+        for (ColourSlot& c : d->slots)
+            if (&c != pick && c.order.in_flight && (!pick || fits(c, n)) && (!oldest || c.turn < oldest->turn)) oldest = &c;
+        if (!pick) pick = oldest;
+        else if (oldest && grow_slot(*pick, n) != cudaSuccess) {
+            (void)cudaGetLastError();
+            pick = oldest;
+        }
+    }
+    pick->turn = ++d->turns;
+    *out = pick;
+    return order_enter(pick->order, st);
+}
+
+bool alloc_frame(ix_backend* b, DisplayState* d, ColourSlot& c, uint64_t n, bool guides_raw, bool xyz, bool rgba) {
     cudaError_t e = grow_device(&d->d_nrm, &d->nrm_cap, n);
     if (e == cudaSuccess) e = grow_device(&d->d_fs, &d->fs_cap, n);
-    if (e == cudaSuccess) e = grow_device(&d->d_col[0], &d->col_cap[0], n);
-    if (e == cudaSuccess) e = grow_device(&d->d_col[1], &d->col_cap[1], n);
+    if (e == cudaSuccess) e = grow_slot(c, n);
     if (e == cudaSuccess && guides_raw) {
         e = grow_device(&d->d_depth, &d->depth_cap, n);
         if (e == cudaSuccess) e = grow_device(&d->d_normal, &d->normal_cap, 3 * n);
@@ -300,11 +360,11 @@ float elapsed(DisplayState* d, int a, int c) {
     return 0.0f;
 }
 
-// The passes over the packed guides in d_nrm / d_fs and the colour in d_col[0]; the last
+// The passes over the packed guides in d_nrm / d_fs and the colour in c.d_col[0]; the last
 // pass writes RGBA8 into `rgba` when it is given, else colour.  Returns the index of the
 // colour buffer holding the result (rgba == null) and counts the launches.
-int run_passes(ix_backend* b, DisplayState* d, const Resolved& r, uint32_t w, uint32_t h, uchar4* rgba,
-               bool facet_normals, uint32_t* launches, cudaError_t* err, cudaStream_t st) {
+int run_passes(ix_backend* b, DisplayState* d, const ColourSlot& c, const Resolved& r, uint32_t w, uint32_t h,
+               uchar4* rgba, bool facet_normals, uint32_t* launches, cudaError_t* err, cudaStream_t st) {
     int cur = 0;
     *err = cudaSuccess;
     for (uint32_t pass = 0; pass < r.passes && *err == cudaSuccess; ++pass) {
@@ -312,12 +372,12 @@ int run_passes(ix_backend* b, DisplayState* d, const Resolved& r, uint32_t w, ui
         L.width = w;
         L.height = h;
         L.stride = 1 << pass;
-        L.src = d->d_col[cur];
+        L.src = c.d_col[cur];
         L.nrm = d->d_nrm;
         L.fs = d->d_fs;
         L.facet_normals = facet_normals ? 1 : 0;
         const bool last = pass + 1 == r.passes;
-        L.dst = (last && rgba) ? nullptr : d->d_col[cur ^ 1];
+        L.dst = (last && rgba) ? nullptr : c.d_col[cur ^ 1];
         L.rgba = (last && rgba) ? rgba : nullptr;
         *err = pass_launch(b, L, st);
         ++*launches;
@@ -327,17 +387,17 @@ int run_passes(ix_backend* b, DisplayState* d, const Resolved& r, uint32_t w, ui
 }
 
 // The frame after packing: identity -> tone-map the average; else the passes with the
-// tone-map fused into the last.  d_col[0] holds the average.
-cudaError_t frame_after_pack(ix_backend* b, DisplayState* d, const Resolved& r, uint32_t w, uint32_t h,
-                             bool facet_normals, uint32_t* launches, cudaStream_t st) {
+// tone-map fused into the last, into `rgba`.  c.d_col[0] holds the average.
+cudaError_t frame_after_pack(ix_backend* b, DisplayState* d, const ColourSlot& c, const Resolved& r, uint32_t w,
+                             uint32_t h, uchar4* rgba, bool facet_normals, uint32_t* launches, cudaStream_t st) {
     const uint64_t n = (uint64_t)w * h;
     if (r.identity) {
-        TonemapLaunch T{n, nullptr, d->d_col[0], 1.0f, IX_COLOR_SPACE_SRGB, d->d_rgba};
+        TonemapLaunch T{n, nullptr, c.d_col[0], 1.0f, IX_COLOR_SPACE_SRGB, rgba};
         ++*launches;
         return tonemap_launch(b, T, st);
     }
     cudaError_t e;
-    run_passes(b, d, r, w, h, d->d_rgba, facet_normals, launches, &e, st);
+    run_passes(b, d, c, r, w, h, rgba, facet_normals, launches, &e, st);
     return e;
 }
 
@@ -408,7 +468,7 @@ int ix_generate_guide_buffers(ix_backend* b, uint32_t width, uint32_t height, co
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     DisplayState* d = state(b);
-    cudaError_t e = order_enter(d->order, b->stream);
+    cudaError_t e = order_all(d, b->stream);
     if (e == cudaSuccess) e = grow_device(&d->d_planes, &d->planes_cap, 4 * (size_t)std::max(n_planes, 1u));
     if (e == cudaSuccess) e = grow_device(&d->d_depth, &d->depth_cap, n);
     if (e == cudaSuccess) e = grow_device(&d->d_normal, &d->normal_cap, 3 * n);
@@ -451,8 +511,9 @@ int ix_atrous_denoise(ix_backend* b, const float* color, const float* depth, con
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     DisplayState* d = state(b);
-    if (fail(b, order_enter(d->order, b->stream), "stream order")) return IX_DECLINED;
-    if (!alloc_frame(b, d, n, true, true, false)) return IX_DECLINED;
+    if (fail(b, order_all(d, b->stream), "stream order")) return IX_DECLINED;
+    ColourSlot& c = d->slots[0];
+    if (!alloc_frame(b, d, c, n, true, true, false)) return IX_DECLINED;
     d->cached = false;
     const auto t0 = std::chrono::steady_clock::now();
     cudaError_t e = h2d_staged(d, d->d_xyz, color, 12 * n, b->stream);
@@ -462,14 +523,14 @@ int ix_atrous_denoise(ix_backend* b, const float* color, const float* depth, con
     if (e == cudaSuccess && path_sig) e = h2d_staged(d, d->d_sig, path_sig, 4 * n, b->stream);
     record(d, 0, b->stream);
     PackLaunch P{n, d->d_depth, d->d_normal, d->d_facet, path_sig ? d->d_sig : nullptr, d->d_nrm, d->d_fs,
-                 d->d_xyz, 1.0f, d->d_col[0]};
+                 d->d_xyz, 1.0f, c.d_col[0]};
     if (e == cudaSuccess) e = launch_pack_exact(P, b->stream);
     record(d, 1, b->stream);
     uint32_t launches = 1;
     int cur = 0;
-    if (e == cudaSuccess) cur = run_passes(b, d, r, width, height, nullptr, false, &launches, &e, b->stream);
+    if (e == cudaSuccess) cur = run_passes(b, d, c, r, width, height, nullptr, false, &launches, &e, b->stream);
     record(d, 2, b->stream);
-    UnpackLaunch U{n, d->d_col[cur], d->d_xyz};
+    UnpackLaunch U{n, c.d_col[cur], d->d_xyz};
     if (e == cudaSuccess) e = unpack_launch(b, U, b->stream);
     ++launches;
     record(d, 3, b->stream);
@@ -491,7 +552,7 @@ static int tonemap_impl(ix_backend* b, const float* xyz, uint64_t pixels, float 
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     DisplayState* d = state(b);
-    cudaError_t e = order_enter(d->order, b->stream);
+    cudaError_t e = order_all(d, b->stream);
     if (e == cudaSuccess) e = grow_device(&d->d_xyz, &d->xyz_cap, 3 * pixels);
     if (e == cudaSuccess) e = grow_device(&d->d_rgba, &d->rgba_cap, pixels);
     if (fail(b, e, "tonemap buffers")) return IX_DECLINED;
@@ -541,8 +602,9 @@ int ix_denoise_and_tonemap_frame(ix_backend* b, uint32_t width, uint32_t height,
     Turn turn(b);
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     DisplayState* d = state(b);
-    if (fail(b, order_enter(d->order, b->stream), "stream order")) return IX_DECLINED;
-    if (!alloc_frame(b, d, n, true, true, true)) return IX_DECLINED;
+    if (fail(b, order_all(d, b->stream), "stream order")) return IX_DECLINED;
+    ColourSlot& c = d->slots[0];
+    if (!alloc_frame(b, d, c, n, true, true, true)) return IX_DECLINED;
     d->cached = false;
     const auto t0 = std::chrono::steady_clock::now();
     cudaError_t e = h2d_staged(d, d->d_xyz, accum, 12 * n, b->stream);
@@ -553,11 +615,11 @@ int ix_denoise_and_tonemap_frame(ix_backend* b, uint32_t width, uint32_t height,
     record(d, 0, b->stream);
     const float inv = 1.0f / (float)spp;
     PackLaunch P{n, d->d_depth, d->d_normal, d->d_facet, path_sig ? d->d_sig : nullptr, d->d_nrm, d->d_fs,
-                 d->d_xyz, inv, d->d_col[0]};
+                 d->d_xyz, inv, c.d_col[0]};
     if (e == cudaSuccess) e = launch_pack_exact(P, b->stream);
     record(d, 1, b->stream);
     uint32_t launches = 1;
-    if (e == cudaSuccess) e = frame_after_pack(b, d, r, width, height, false, &launches, b->stream);
+    if (e == cudaSuccess) e = frame_after_pack(b, d, c, r, width, height, d->d_rgba, false, &launches, b->stream);
     record(d, 2, b->stream);
     if (e == cudaSuccess) e = d2h_staged(d, rgba, d->d_rgba, 4 * n, b->stream);
     if (fail(b, e, "denoise and tonemap")) return IX_DECLINED;
@@ -593,8 +655,9 @@ static int display_frame_impl(ix_backend* b, const ix_scene* scene, uint32_t wit
     if (fail(b, cudaSetDevice(b->device), "set device")) return IX_DECLINED;
     const cudaStream_t st = stream ? stream : b->stream;
     DisplayState* d = state(b);
-    if (fail(b, order_enter(d->order, st), "stream order")) return IX_DECLINED;
-    if (!alloc_frame(b, d, n, false, accum_dev == nullptr, rgba_dev == nullptr)) return IX_DECLINED;
+    ColourSlot* slot = &d->slots[0];
+    if (fail(b, rgba_host ? order_all(d, st) : take_slot(d, n, st, &slot), "stream order")) return IX_DECLINED;
+    if (!alloc_frame(b, d, *slot, n, false, accum_dev == nullptr, rgba_dev == nullptr)) return IX_DECLINED;
     if (fail(b, grow_device(&d->d_planes, &d->planes_cap, 4 * (size_t)std::max(sc.n_planes, 1u)), "planes"))
         return IX_DECLINED;
     const auto t0 = std::chrono::steady_clock::now();
@@ -606,13 +669,17 @@ static int display_frame_impl(ix_backend* b, const ix_scene* scene, uint32_t wit
     if (!d->cached || key != d->cache_key) {
         // The guides depend only on the camera pose and the facet geometry (guide_pass.rs
         // module docs): computed once per pose, reused for every frame of it.
-        e = h2d(d->d_planes, sc.planes, 16 * (size_t)sc.n_planes, st);
+        e = order_all(d, st);  // frames in flight read the guides of another
+        if (e == cudaSuccess) e = h2d(d->d_planes, sc.planes, 16 * (size_t)sc.n_planes, st);
         GuideLaunch G{sc.camera, sc.width, sc.height, reinterpret_cast<const float4*>(d->d_planes), sc.n_planes, n_d,
                       nullptr, nullptr, nullptr, nullptr, d->d_nrm, d->d_fs};
         if (e == cudaSuccess) e = launch_guides_exact(G, st);
         ++launches;
+        if (!rgba_host && e == cudaSuccess) e = order_leave(d->guides, st);
         d->cached = e == cudaSuccess;
         d->cache_key = key;
+    } else if (capturing(st) || !order_idle(d->guides)) {
+        e = order_enter(d->guides, st);
     }
     record(d, 1, st);
     const float* src = accum_dev;
@@ -623,24 +690,21 @@ static int display_frame_impl(ix_backend* b, const ix_scene* scene, uint32_t wit
     record(d, 2, st);
     if (spp == 0) {
         // rgba_dev only: the tone-map of zeros.
-        if (e == cudaSuccess) e = cudaMemsetAsync(d->d_col[0], 0, 16 * n, st);
-        TonemapLaunch T{n, nullptr, d->d_col[0], 1.0f, IX_COLOR_SPACE_SRGB, reinterpret_cast<uchar4*>(rgba_dev)};
+        if (e == cudaSuccess) e = cudaMemsetAsync(slot->d_col[0], 0, 16 * n, st);
+        TonemapLaunch T{n, nullptr, slot->d_col[0], 1.0f, IX_COLOR_SPACE_SRGB, reinterpret_cast<uchar4*>(rgba_dev)};
         if (e == cudaSuccess) e = tonemap_launch(b, T, st);
         ++launches;
     } else {
         const float inv = 1.0f / (float)spp;
-        PackLaunch P{n, nullptr, nullptr, nullptr, nullptr, d->d_nrm, nullptr, src, inv, d->d_col[0]};
+        PackLaunch P{n, nullptr, nullptr, nullptr, nullptr, d->d_nrm, nullptr, src, inv, slot->d_col[0]};
         if (e == cudaSuccess) e = launch_pack_exact(P, st);
         ++launches;
         uchar4* out = rgba_dev ? reinterpret_cast<uchar4*>(rgba_dev) : d->d_rgba;
-        uchar4* keep = d->d_rgba;
-        d->d_rgba = out;
-        if (e == cudaSuccess) e = frame_after_pack(b, d, r, sc.width, sc.height, true, &launches, st);
-        d->d_rgba = keep;
+        if (e == cudaSuccess) e = frame_after_pack(b, d, *slot, r, sc.width, sc.height, out, true, &launches, st);
     }
     record(d, 3, st);
     // The host form waits for its RGBA8; the device form stays asynchronous on `st`.
-    if (!rgba_host && e == cudaSuccess) e = order_leave(d->order, st);
+    if (!rgba_host && e == cudaSuccess) e = order_leave(slot->order, st);
     if (rgba_host && e == cudaSuccess) e = d2h_staged(d, rgba_host, d->d_rgba, 4 * n, st);
     if (fail(b, e, "display frame")) {
         d->cached = false;

@@ -53,6 +53,35 @@ def test_displayed_frames_on_two_streams(backend, w, h, same_view):
     assert np.array_equal(np.asarray(host).reshape(h, w, 4), want[0].cpu().numpy())
 
 
+def test_more_streams_than_colour_buffers(backend):
+    import torch
+
+    w, h = 200, 120
+    g = torch.Generator(device="cuda").manual_seed(3)
+    views = [_view(0.6, w, h).to_abi(), _view(2.2, w, h).to_abi()]
+    sums = [torch.rand(h, w, 3, device="cuda", generator=g) * 16.0 for _ in range(7)]
+
+    def show(i, view, out, stream):
+        assert display.display_frame_device(backend, views[view], 16, sums[i].data_ptr(), out.data_ptr(), False,
+                                            stream_ptr=stream.cuda_stream if stream else None)
+
+    want = torch.zeros(2, 7, h, w, 4, dtype=torch.uint8, device="cuda")
+    for view in range(2):
+        for i in range(7):
+            torch.cuda.synchronize()
+            show(i, view, want[view, i], None)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(6)] + [None]
+    got = torch.zeros(12, 7, h, w, 4, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    for k in range(12):  # the view changes while frames of the other are in flight
+        for i in range(7):
+            show(i, k // 3 % 2, got[k, i], streams[(i + k) % 7])
+    torch.cuda.synchronize()
+    for k in range(12):
+        assert torch.equal(got[k], want[k // 3 % 2])
+
+
 def test_traced_frames_on_two_streams(backend):
     import torch
 
