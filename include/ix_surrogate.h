@@ -25,6 +25,12 @@ extern "C" {
  * k x m); op(B) = B (k x n, ldb) or B^T when trans_b (B is n x k).  BF16 operands. */
 int ix_mlp_gemm_bf16(int trans_a, int trans_b, uint32_t m, uint32_t n, uint32_t k, const void* a, uint32_t lda,
                      const void* b, uint32_t ldb, float* c, uint32_t ldc, void* stream);
+/* The same with the caller's memory for the partial sums of a product split over K:
+ * IX_MLP_GEMM_WORKSPACE floats that no other call uses until this one is done (NULL: the call
+ * takes its own from a pool, in the stream's order). */
+#define IX_MLP_GEMM_WORKSPACE (148 * 128 * 32)
+int ix_mlp_gemm_bf16_ws(int trans_a, int trans_b, uint32_t m, uint32_t n, uint32_t k, const void* a, uint32_t lda,
+                        const void* b, uint32_t ldb, float* c, uint32_t ldc, float* workspace, void* stream);
 /* One dense layer, y = x W^T + bias with x (m x k, ldx, bf16) and W (n x k, bf16): z = y
  * (f32, pre-activation), h = silu(y) when silu_act else y (f32), hb = bf16(h); any of z,
  * h, hb may be NULL; bias may be NULL (zero).  z, h, hb are m x n, row stride n. */

@@ -426,11 +426,13 @@ cudaError_t launch_nt(const GemmParams& p, uint32_t splits, int device, cudaStre
 
 __device__ unsigned int g_umma_status;
 
-// Where the split-K partials live: each call takes its own stretch of a pool of its device, in
-// its stream's order, and gives it back behind its sum, so that calls on other streams or from
-// other threads never share one.  A call needs at most SM_COUNT tiles of 128 x 32 f32 (2.4 MB:
-// what splits has the narrowest tile); the pool holds on to KEEP_BYTES between calls at most
-// and returns the rest to the device at the next synchronisation.
+// Where the split-K partials live: in the caller's workspace, or else in a stretch of a pool of
+// the device that the call takes in its stream's order and gives back behind its sum, so that
+// calls on other streams or from other threads never share one.  A call needs at most SM_COUNT
+// tiles of 128 x 32 f32 (2.4 MB: what splits has the narrowest tile); the pool holds on to
+// KEEP_BYTES between calls at most and returns the rest to the device at the next
+// synchronisation.  Taking and giving back costs the host 3 us a call.
+static_assert(IX_MLP_GEMM_WORKSPACE == SM_COUNT * TM * 32, "the narrowest tile");
 constexpr uint64_t KEEP_BYTES = 64ull << 20;
 std::mutex g_pools_mu;
 cudaMemPool_t g_pools[MAX_DEVICES];
@@ -444,6 +446,9 @@ cudaMemPool_t partials_pool(int device) {
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
     uint64_t keep = KEEP_BYTES;
+    // The first call may be a captured one: the pool is no part of the capture.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
     if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
         pool = nullptr;
     } else if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
@@ -451,12 +456,13 @@ cudaMemPool_t partials_pool(int device) {
         pool = nullptr;
     }
     if (!pool) (void)cudaGetLastError();
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
     return pool;
 }
 
 uint32_t tiles(uint32_t x, uint32_t t) { return (x + t - 1) / t; }
 
-int run(GemmParams p, void* stream) {
+int run(GemmParams p, void* stream, float* workspace = nullptr) {
     if (p.m == 0 || p.n == 0) return 0;
     if (p.k == 0 || !p.a || !p.b) return 1;
     if (p.m > (1u << 30) || p.n > (1u << 30) || p.k > (1u << 30)) return 1;
@@ -490,8 +496,8 @@ int run(GemmParams p, void* stream) {
     if (splits > 1) splits = tiles(p.k, p.k_split);  // every split non-empty
     float* c = p.out_f32;
     const uint32_t ldc = p.ldo;
-    float* partials = nullptr;
-    if (splits > 1) {
+    float* partials = nullptr;  // of the pool
+    if (splits > 1 && !workspace) {
         const cudaMemPool_t pool = partials_pool(device);
         if (!pool) return 1;
         if (cudaMallocFromPoolAsync((void**)&partials, (size_t)splits * p.m * p.n * sizeof(float), pool, s) !=
@@ -499,7 +505,9 @@ int run(GemmParams p, void* stream) {
             (void)cudaGetLastError();
             return 1;
         }
-        p.out_f32 = partials;
+    }
+    if (splits > 1) {
+        p.out_f32 = workspace ? workspace : partials;
         p.ldo = p.n;
         p.out_bf16 = nullptr;
     }
@@ -530,6 +538,11 @@ extern "C" {
 
 int ix_mlp_gemm_bf16(int trans_a, int trans_b, uint32_t m, uint32_t n, uint32_t k, const void* a, uint32_t lda,
                      const void* b, uint32_t ldb, float* c, uint32_t ldc, void* stream) {
+    return ix_mlp_gemm_bf16_ws(trans_a, trans_b, m, n, k, a, lda, b, ldb, c, ldc, nullptr, stream);
+}
+
+int ix_mlp_gemm_bf16_ws(int trans_a, int trans_b, uint32_t m, uint32_t n, uint32_t k, const void* a, uint32_t lda,
+                        const void* b, uint32_t ldb, float* c, uint32_t ldc, float* workspace, void* stream) {
     // C = op(A) op(B) in the kernel's form C = A' B'^T: A'(r, kk) = op(A)(r, kk) and
     // B'(col, kk) = op(B)(kk, col).
     if (!c) return 1;
@@ -546,7 +559,7 @@ int ix_mlp_gemm_bf16(int trans_a, int trans_b, uint32_t m, uint32_t n, uint32_t 
     p.epi = EPI_STORE;
     p.out_f32 = c;
     p.ldo = ldc;
-    return run(p, stream);
+    return run(p, stream, workspace);
 }
 
 int ix_mlp_linear(uint32_t m, uint32_t n, uint32_t k, const void* x, uint32_t ldx, const void* w, const float* bias,

@@ -42,6 +42,7 @@ TILTS_DEG = (0.0, 5.0, 10.0, 15.0, 20.0, 25.0, 30.0, 35.0, 40.0)
 METRICS = ("brilliance", "fire", "scintillation")
 N_OUTPUTS = len(METRICS) * len(TILTS_DEG)  # output k = metric k // 9 at tilt k % 9
 DIMS = (N_FEATURES, 256, 256, 256, N_OUTPUTS)
+GEMM_WORKSPACE = 148 * 128 * 32  # IX_MLP_GEMM_WORKSPACE (include/ix_surrogate.h)
 FACE_UP_DISTANCE = 1.6
 FOV_DEG = 42.0
 
@@ -77,6 +78,7 @@ def _lib() -> C.CDLL:
         vp = C.c_void_p
         u32, u64, f32 = C.c_uint32, C.c_uint64, C.c_float
         lib.ix_mlp_gemm_bf16.argtypes = [C.c_int, C.c_int, u32, u32, u32, vp, u32, vp, u32, vp, u32, vp]
+        lib.ix_mlp_gemm_bf16_ws.argtypes = lib.ix_mlp_gemm_bf16.argtypes[:-1] + [vp, vp]
         lib.ix_mlp_linear.argtypes = [u32, u32, u32, vp, u32, vp, vp, C.c_int, vp, vp, vp, vp]
         lib.ix_mlp_backward_silu.argtypes = [u32, u32, u32, vp, vp, vp, vp, vp, vp]
         lib.ix_mlp_status.argtypes = [C.c_int]
@@ -292,13 +294,15 @@ class SurrogateMLP:
         _ok(lib.ix_mlp_mse_grad(m, out.shape[1], out.data_ptr(), tt.data_ptr(), d_f32.data_ptr(), d_b16.data_ptr(),
                                 loss.data_ptr(), s))
         grads = [None] * len(self.layers)
+        ws = torch.empty(GEMM_WORKSPACE, dtype=torch.float32, device=self.dev)
         for li in range(len(self.layers) - 1, -1, -1):
             L = self.layers[li]
             h_in = acts[li][0]
             n, k = L.w.shape
             # dW = dZ^T h_in: (n x m) (m x k).
             dw = torch.empty(n, k, dtype=torch.float32, device=self.dev)
-            _ok(lib.ix_mlp_gemm_bf16(1, 0, n, k, m, d_b16.data_ptr(), n, h_in.data_ptr(), k, dw.data_ptr(), k, s))
+            _ok(lib.ix_mlp_gemm_bf16_ws(1, 0, n, k, m, d_b16.data_ptr(), n, h_in.data_ptr(), k, dw.data_ptr(), k,
+                                        ws.data_ptr(), s))
             db = torch.empty(n, dtype=torch.float32, device=self.dev)
             _ok(lib.ix_mlp_bias_grad(m, n, d_f32.data_ptr(), db.data_ptr(), s))
             grads[li] = (dw, db)

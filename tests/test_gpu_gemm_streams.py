@@ -90,3 +90,21 @@ def test_a_captured_weight_gradient_replays_on_new_operands():
         call(eager)
         assert torch.equal(dw, eager)
     assert lib.ix_mlp_status(1) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(256, 256, 4096), (27, 256, 4096), (128, 32, 8192), (128, 128, 16384),
+                                   (9344, 32, 1024), (256, 12, 513), (64, 64, 64)])
+def test_a_workspace_gives_the_same_bits(m, n, k):
+    """The caller's workspace: the pool's sums, and nothing past IX_MLP_GEMM_WORKSPACE floats."""
+    import torch
+
+    lib, s = surrogate._lib(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn(k, m, device="cuda", generator=g).bfloat16()
+    b = torch.randn(k, n, device="cuda", generator=g).bfloat16()
+    want, got = torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda")
+    ws = torch.full((surrogate.GEMM_WORKSPACE + 4096,), 7.0, device="cuda")
+    assert lib.ix_mlp_gemm_bf16(1, 0, m, n, k, a.data_ptr(), m, b.data_ptr(), n, want.data_ptr(), n, s) == 0
+    assert lib.ix_mlp_gemm_bf16_ws(1, 0, m, n, k, a.data_ptr(), m, b.data_ptr(), n, got.data_ptr(), n, ws.data_ptr(),
+                                   s) == 0
+    assert torch.equal(got, want) and bool((ws[surrogate.GEMM_WORKSPACE:] == 7.0).all())
