@@ -466,17 +466,22 @@ int run(GemmParams p, void* stream, float* workspace = nullptr) {
     if (p.m == 0 || p.n == 0) return 0;
     if (p.k == 0 || !p.a || !p.b) return 1;
     if (p.m > (1u << 30) || p.n > (1u << 30) || p.k > (1u << 30)) return 1;
-    void* st_ptr = nullptr;
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device >= MAX_DEVICES) {
         (void)cudaGetLastError();
         return 1;
     }
-    if (cudaGetSymbolAddress(&st_ptr, g_umma_status) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return 1;
+    static std::atomic<unsigned int*> status[MAX_DEVICES];  // the word's address on each
+    p.status = status[device].load(std::memory_order_acquire);
+    if (!p.status) {
+        void* address = nullptr;
+        if (cudaGetSymbolAddress(&address, g_umma_status) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return 1;
+        }
+        p.status = static_cast<unsigned int*>(address);
+        status[device].store(p.status, std::memory_order_release);
     }
-    p.status = static_cast<unsigned int*>(st_ptr);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // Tile width: the narrowest of 32 / 64 / 128 / 256 that covers n, halved (down to 32)
     // while the grid would give fewer than two CTAs per SM.
